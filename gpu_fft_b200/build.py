@@ -9,16 +9,22 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgpufft_b200.so")
 
-SOURCES = ["gpufft.cu", "fast_f32.cu", "fast_f64.cu", "noalloc.cu", "batch.cu", "s16.cu", "serve.cu", "dist.cu", "fast_f32_3s.cu", "hostpipe.cu", "fast_queue.cu"]
-HEADERS = ["fft_kernels.cuh", "fft_radix.cuh", "fft_fast.cuh", "fft_s16.cuh", "fft_queue.cuh", "fast_registry.h", "fast_entries.h", "gpufft_internal.h"]
+SOURCES = ["gpufft.cu", "fast_f32.cu", "fast_f64.cu", "noalloc.cu", "batch.cu", "s16.cu", "serve.cu", "dist.cu", "fast_f32_3s.cu", "hostpipe.cu", "fast_queue.cu",
+           "axis.cu", "axis_cols_f32.cu", "axis_cols_epi_f32.cu", "axis_rows_f32.cu", "axis_cols_f64.cu",
+           "axis_cols_epi_f64.cu", "axis_rows_f64.cu"]
+# sources compiled several times: (source, object name, definitions)
+PARTS = [("axis_fixed.cu", f"axis_fixed_{d}_{i}.o", [f"-DGPUFFT_AXIS_F64={d}", f"-DGPUFFT_AXIS_PART={i}"])
+         for d in (1, 0) for i in range(8)]
+HEADERS = ["fft_axis.cuh", "axis_lengths.h", "fft_kernels.cuh", "fft_radix.cuh", "fft_fast.cuh", "fft_s16.cuh", "fft_queue.cuh", "fast_registry.h", "fast_entries.h", "gpufft_internal.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
+FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2", "-Xfatbin=-compress-all"]
 
 
 def nvcc() -> str:
@@ -27,7 +33,7 @@ def nvcc() -> str:
 
 
 def _inputs() -> list[str]:
-    files = [os.path.join(CSRC, f) for f in SOURCES + HEADERS]
+    files = [os.path.join(CSRC, f) for f in SOURCES + HEADERS + [p[0] for p in PARTS]]
     files.append(os.path.join(ROOT, "include", "gpufft_b200.h"))
     return files
 
@@ -45,16 +51,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
-    procs, objs = [], []
-    for f in SOURCES:
-        obj = os.path.join(objdir, f.replace(".cu", ".o"))
-        objs.append(obj)
-        cmd = [nvcc(), *ARCH, *FLAGS, "-c", "-o", obj, os.path.join(CSRC, f)]
+    jobs = PARTS + [(f, f.replace(".cu", ".o"), []) for f in SOURCES]
+
+    def compile_one(job):
+        src, obj, defs = job
+        cmd = [nvcc(), *ARCH, *FLAGS, *defs, "-c", "-o", os.path.join(objdir, obj), os.path.join(CSRC, src)]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
             print(" ".join(cmd))
-        procs.append((f, subprocess.Popen(cmd)))
-    failed = [f for f, p in procs if p.wait() != 0]
+        return subprocess.run(cmd).returncode
+
+    with ThreadPoolExecutor(max_workers=max(2, os.cpu_count() or 2)) as pool:
+        failed = [job[1] for job, rc in zip(jobs, pool.map(compile_one, jobs)) if rc != 0]
+    objs = [os.path.join(objdir, job[1]) for job in jobs]
     if failed:
         raise RuntimeError(f"nvcc failed on {failed}")
     subprocess.run([nvcc(), *ARCH, "-shared", "-o", LIB + ".tmp", *objs, "-lcudart", "-ldl"], check=True)

@@ -513,6 +513,10 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
         const long long tiles = (ncols + P.fb->w - 1) / P.fb->w;
         P.grid_fb = (int)std::min<long long>(tiles, (long long)P.occ_fb * sms);
     }
+    if (!P.fa || (!P.fb && !P.tc_split)) {
+        const int ra = axis::form_create(P);
+        if (ra != GPUFFT_SUCCESS) return ra;
+    }
     return P.dtype == GPUFFT_FLOAT ? upload_stage_tables<float>(P) : upload_stage_tables<double>(P);
 }
 
@@ -828,7 +832,7 @@ static int build_plan(Plan &P) {
     P.occ_b = occ_b;
     if (std::getenv("GPUFFT_GENERIC_ONLY") && !P.tc_split) {
         P.idx_a = P.idx_b = -1;
-        return GPUFFT_SUCCESS;
+        return axis::form_create(P);
     }
     int ia = 0, ib = 0;
     if (wisdom_lookup(P, ia, ib, P.kfix)) P.tuned = true;
@@ -895,6 +899,7 @@ int plan_destroy(Plan *P) {
         cudaFree(P->tw_dev);
         if (P->stage_dev) cudaFree(P->stage_dev);
         free_queue(*P);
+        axis::form_destroy(*P);
         if (cur != P->device && cur >= 0) cudaSetDevice(cur);
     }
     delete P;
@@ -992,6 +997,7 @@ static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, co
         const cudaError_t e = cudaLaunchKernelExC(&cfg, fwd ? kf : ki, args);
         return e == cudaSuccess ? GPUFFT_SUCCESS : cuda_error(e, "launch pass A (specialised)");
     }
+    if (!P.fa && !xch && axis::has_a(P)) return axis::launch_a(P, data, s, fwd);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(P.grid_a, 1, 1);
@@ -1039,6 +1045,7 @@ static int launch_pass_b(const Plan &P, void *data, cudaStream_t s, bool fwd, do
         const cudaError_t e = cudaLaunchKernel(k, dim3(P.grid_fb), dim3(P.fb->nt), args, P.fb->smem, s);
         return e == cudaSuccess ? GPUFFT_SUCCESS : cuda_error(e, "launch pass B (specialised)");
     }
+    if (!P.fb && axis::has_b(P)) return axis::launch_b(P, data, s, fwd, scale, dealias);
     if (fwd)
         pass_b_kernel<T, true><<<P.grid_b, kThreads, P.smem_b, s>>>(prm);
     else
@@ -1110,7 +1117,7 @@ int plan_exec_pass_a_xch(const Plan *P, void *data, void *xch, int nyl, long lon
                                     : launch_pass_a<double>(*P, data, s, forward, &x);
 }
 
-int plan_launches(const Plan *P) { return P ? (P->nx == 1 ? 1 : 2) + (P->fa && P->split_a ? 1 : 0) : 0; }
+int plan_launches(const Plan *P) { return P ? (P->nx == 1 ? 1 : 2) + ((P->fa ? P->split_a : axis::has_a(*P)) ? 1 : 0) : 0; }
 
 static void describe_axis(std::string &out, const char *name, const AxisPlan &ax) {
     char b[64];
@@ -1153,6 +1160,7 @@ int plan_describe(const Plan *P, char *buf, int len) {
                  P->fb->nt, P->fb->v, P->grid_fb, P->occ_fb, P->fb->smem);
         s += b;
     }
+    axis::form_describe(*P, s, !P->fa, !P->fb);
     if (buf && len > 0) {
         strncpy(buf, s.c_str(), (size_t)len - 1);
         buf[len - 1] = 0;

@@ -3,6 +3,7 @@
 #include <cstdarg>
 #include <cstddef>
 #include <cstdint>
+#include <string>
 
 #include <cuda_runtime.h>
 
@@ -10,6 +11,10 @@
 #include "fft_kernels.cuh"
 
 namespace gpufft {
+
+namespace axis {
+struct Form;
+}
 
 struct Plan {
     int64_t nx = 0, ny = 0, nz = 0;
@@ -43,7 +48,21 @@ struct Plan {
     const void *q_unp = nullptr;    // forward unpack factors
     const void *q_unp_i = nullptr;  // inverse pack factors
     const void *q_rtw = nullptr;  // the row FFT's step-1 twiddles
+    // one-axis-per-launch kernels (axis.cu), made when a pass has no specialised kernel
+    axis::Form *axis = nullptr;
 };
+
+namespace axis {
+// Makes P.axis (once): what the passes of this grid need, for those of its
+// lengths that fft_axis.cuh takes (has_a: the z and y axes, has_b: the x axis).
+int form_create(Plan &P);
+void form_destroy(Plan &P);
+bool has_a(const Plan &P);
+bool has_b(const Plan &P);
+int launch_a(const Plan &P, void *data, cudaStream_t s, bool fwd);
+int launch_b(const Plan &P, void *data, cudaStream_t s, bool fwd, double scale, int dealias);
+void form_describe(const Plan &P, std::string &out, bool a, bool b);
+}  // namespace axis
 
 int set_error(int code, const char *fmt, ...);
 const char *last_error();
