@@ -17,11 +17,10 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgpufft_b200.so")
 
 SOURCES = ["gpufft.cu", "fast_f32.cu", "fast_f64.cu", "noalloc.cu", "batch.cu", "s16.cu", "serve.cu", "dist.cu", "fast_f32_3s.cu", "hostpipe.cu", "fast_queue.cu",
-           "axis.cu", "axis_cols_f32.cu", "axis_cols_epi_f32.cu", "axis_rows_f32.cu", "axis_cols_f64.cu",
-           "axis_cols_epi_f64.cu", "axis_rows_f64.cu"]
+           "axis.cu"]
 # sources compiled several times: (source, object name, definitions)
-PARTS = [("axis_fixed.cu", f"axis_fixed_{d}_{i}.o", [f"-DGPUFFT_AXIS_F64={d}", f"-DGPUFFT_AXIS_PART={i}"])
-         for d in (1, 0) for i in range(8)]
+PARTS = [("axis_kernels.cu", f"axis_kernels_{d}_{i}.o", [f"-DGPUFFT_AXIS_F64={d}", f"-DGPUFFT_AXIS_PART={i}"])
+         for d in (1, 0) for i in range(16)]
 HEADERS = ["fft_axis.cuh", "axis_lengths.h", "fft_kernels.cuh", "fft_radix.cuh", "fft_fast.cuh", "fft_s16.cuh", "fft_queue.cuh", "fast_registry.h", "fast_entries.h", "gpufft_internal.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2", "-Xfatbin=-compress-all"]

@@ -396,7 +396,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // A 2D view of the field in 8-byte elements: `width` elements per line,
 // `lines` lines `pitch` bytes apart, boxes of box_w x box_h.
-static bool encode_view(CUtensorMap *m, void *data, long long width, long long lines, long long pitch, int box_w,
+bool encode_view(CUtensorMap *m, void *data, long long width, long long lines, long long pitch, int box_w,
                         int box_h) {
     const auto enc = tensor_map_encoder();
     if (!enc) return false;

@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <string>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "fast_registry.h"
@@ -70,6 +71,8 @@ const char *last_error();
 // least `bytes`.  Never lowers it: plans of different sizes share the generic
 // kernels, and a later, smaller plan must not undo an earlier plan's limit.
 cudaError_t raise_smem_limit(const void *fn, size_t bytes);
+// tensor map of a 2D view in 8-byte elements (gpufft.cu)
+bool encode_view(CUtensorMap *m, void *data, long long width, long long lines, long long pitch, int box_w, int box_h);
 // slab-decomposed plans (dist.cu), for the reference-shaped process-wide plans
 struct DistPlan;
 int dist_exec(DistPlan *D, void *data, cudaStream_t s, bool fwd);
