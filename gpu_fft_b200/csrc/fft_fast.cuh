@@ -612,13 +612,15 @@ __device__ __forceinline__ void pass_b_fast_run(const PassBParams &P, unsigned c
         const long long c0 = t * W;
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = base + c0;
+        static_assert(NT % W == 0, "a thread's elements are of one column");
+        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
         auto src = [&](int n, int w) -> V {
             return (w < wv) ? ld_g(g + (long long)n * ncols + w) : V{(T)0, (T)0};
         };
         auto dst = [&](int n, int w, V v) {
             if (w < wv) {
                 if constexpr (EPI)
-                    st_g(g + (long long)n * ncols + w, pass_b_epilogue(P, v, n, c0 + w));
+                    st_g(g + (long long)n * ncols + w, epi(v, n));
                 else
                     st_g(g + (long long)n * ncols + w, v);
             }
@@ -706,10 +708,12 @@ __global__ void __launch_bounds__(NT, MINB) pass_b_pipe(PassBParams P) {
         const long long c0 = t * W;
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = obase + c0;
+        static_assert(NT % W == 0, "a thread's elements are of one column");
+        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
         auto dst = [&](int n, int w, V v) {
             if (w < wv) {
                 if constexpr (EPI)
-                    st_g(g + (long long)n * ncols + w, pass_b_epilogue(P, v, n, c0 + w));
+                    st_g(g + (long long)n * ncols + w, epi(v, n));
                 else
                     st_g(g + (long long)n * ncols + w, v);
             }
@@ -764,10 +768,12 @@ __global__ void __launch_bounds__(NT, MINB) pass_b_pipe1(PassBParams P) {
         const long long c0 = t * W;
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = obase + c0;
+        static_assert(NT % W == 0, "a thread's elements are of one column");
+        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
         auto dst = [&](int n, int w, V v) {
             if (w < wv) {
                 if constexpr (EPI)
-                    st_g(g + (long long)n * ncols + w, pass_b_epilogue(P, v, n, c0 + w));
+                    st_g(g + (long long)n * ncols + w, epi(v, n));
                 else
                     st_g(g + (long long)n * ncols + w, v);
             }

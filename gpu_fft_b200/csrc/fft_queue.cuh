@@ -753,10 +753,12 @@ __global__ void __launch_bounds__(NT, 1) pass_b_tma(const PassBParams P, const _
         const long long c0 = t * W;
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = base + c0;
+        static_assert(NT % W == 0, "a thread's elements are of one column");
+        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
         auto dst = [&](int n, int w, V v) {
             if (w < wv) {
                 if constexpr (EPI)
-                    st_g(g + (long long)n * ncols + w, pass_b_epilogue(P, v, n, c0 + w));
+                    st_g(g + (long long)n * ncols + w, epi(v, n));
                 else
                     st_g(g + (long long)n * ncols + w, v);
             }
