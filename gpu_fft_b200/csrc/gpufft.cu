@@ -427,6 +427,7 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
     const int sms = device_sms(P.device);
     P.fa = nullptr;
     P.fb = nullptr;
+    P.axis_a = P.axis_b = false;
     P.idx_a = idx_a;
     P.idx_b = idx_b;
     int seen = 0;
@@ -518,6 +519,36 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
         if (ra != GPUFFT_SUCCESS) return ra;
     }
     return P.dtype == GPUFFT_FLOAT ? upload_stage_tables<float>(P) : upload_stage_tables<double>(P);
+}
+
+// Plans that name no candidate (no autotuning, wisdom or variable) take the
+// one-axis-per-launch kernels over the registered ones where they measured
+// faster (ms per launch or pair of launches, forward + inverse):
+//  * Pass A: the queue form stays at 512^2 planes (512^3 FP32 0.72 against
+//    0.86, FP64 1.50 against 1.58) and goes at 512 x 128 (FP32 0.89 against
+//    0.86, FP64 1.88 against 1.58) and 360 x 240 (0.45 against 0.42, FP64 0.86
+//    against 0.85).  The cluster forms stay for fields of up to 3 MB, where one
+//    launch instead of two is what counts (64^3 0.012 against 0.020; 96^3, 3.6
+//    MB, 0.029 against 0.023; 256^3 0.167 against 0.118; 1024^3 9.68 against
+//    7.51).
+//  * x pass: the tensor-copy form stays (512^3 FP32 0.371 against 0.399), as
+//    do short axes and the double-buffered tiles of 128 and 256 points in
+//    FP32 (128 x 512 x 512 0.104 against 0.121); the others go (288^3 0.092
+//    against 0.070, 486^3 0.535 against 0.336, 1024 x 512 x 256 0.447 against
+//    0.396, 128 x 512 x 512 FP64 0.304 against 0.203).
+static int prefer_axis(Plan &P, bool pick_a, bool pick_b) {
+    const double bytes = (double)P.nx * P.ny * (P.nz / 2 + 1) * (P.dtype == GPUFFT_FLOAT ? 8 : 16);
+    bool a = false, b = false;
+    if (pick_a && P.fa) a = P.fa->kind == 2 ? P.fa->m != 256 : bytes > 3e6;
+    if (pick_b && P.fb && !P.tc_split)
+        b = P.fb->kind != 3 && P.nx >= 96 &&
+            !(P.dtype == GPUFFT_FLOAT && P.fb->kind == 1 && (P.nx == 128 || P.nx == 256));
+    if (!a && !b) return GPUFFT_SUCCESS;
+    const int rc = axis::form_create(P);
+    if (rc != GPUFFT_SUCCESS) return rc;
+    P.axis_a = a && axis::has_a(P);
+    P.axis_b = b && axis::has_b(P);
+    return GPUFFT_SUCCESS;
 }
 
 // ---------------------------------------------------------------------------
@@ -839,7 +870,8 @@ static int build_plan(Plan &P) {
     const char *va = std::getenv("GPUFFT_VARIANT_A"), *vb = std::getenv("GPUFFT_VARIANT_B");
     if (va) ia = std::atoi(va);
     if (vb) ib = std::atoi(vb);
-    const int rc = setup_fast(P, ia, ib);
+    int rc = setup_fast(P, ia, ib);
+    if (rc == GPUFFT_SUCCESS) rc = prefer_axis(P, !P.tuned && !va, !P.tuned && !vb);
     if (rc == GPUFFT_SUCCESS && P.tc_split && !P.fb)
         return set_error(GPUFFT_ERR_UNSUPPORTED,
                          "no tensor-core x-pass kernel for Nx=%lld (compiled: FP32, Nx = 512 and 1024)", (long long)nx);
@@ -885,8 +917,12 @@ int plan_adopt(Plan *P, const Plan *Q) {
         return set_error(GPUFFT_ERR_INVALID, "plan_adopt: the plans differ in grid or form");
     if (Q->idx_a < 0 && Q->idx_b < 0) return GPUFFT_SUCCESS;  // generic kernels: nothing to copy
     P->kfix = Q->kfix;
-    const int rc = setup_fast(*P, Q->idx_a, Q->idx_b);
-    if (rc == GPUFFT_SUCCESS) P->tuned = Q->tuned;
+    int rc = setup_fast(*P, Q->idx_a, Q->idx_b);
+    if (rc == GPUFFT_SUCCESS && (Q->axis_a || Q->axis_b)) rc = axis::form_create(*P);
+    if (rc != GPUFFT_SUCCESS) return rc;
+    P->axis_a = Q->axis_a;
+    P->axis_b = Q->axis_b;
+    P->tuned = Q->tuned;
     return rc;
 }
 
@@ -916,6 +952,7 @@ struct XchLayout {
 
 template <typename T>
 static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, const XchLayout *xch = nullptr) {
+    if ((!P.fa || P.axis_a) && !xch && axis::has_a(P)) return axis::launch_a(P, data, s, fwd);
     PassAParams prm = P.pa;
     prm.data = data;
     const void *kf = P.fa ? P.fa->kfwd : nullptr, *ki = P.fa ? P.fa->kinv : nullptr;
@@ -997,7 +1034,6 @@ static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, co
         const cudaError_t e = cudaLaunchKernelExC(&cfg, fwd ? kf : ki, args);
         return e == cudaSuccess ? GPUFFT_SUCCESS : cuda_error(e, "launch pass A (specialised)");
     }
-    if (!P.fa && !xch && axis::has_a(P)) return axis::launch_a(P, data, s, fwd);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = dim3(P.grid_a, 1, 1);
@@ -1018,6 +1054,7 @@ static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, co
 template <typename T>
 static int launch_pass_b(const Plan &P, void *data, cudaStream_t s, bool fwd, double scale = 1.0, int dealias = 0) {
     if (P.nx == 1) return GPUFFT_SUCCESS;  // a length-1 DFT is the identity
+    if ((!P.fb || P.axis_b) && axis::has_b(P)) return axis::launch_b(P, data, s, fwd, scale, dealias);
     PassBParams prm = P.pb;
     prm.data = data;
     prm.scale = scale;
@@ -1045,7 +1082,6 @@ static int launch_pass_b(const Plan &P, void *data, cudaStream_t s, bool fwd, do
         const cudaError_t e = cudaLaunchKernel(k, dim3(P.grid_fb), dim3(P.fb->nt), args, P.fb->smem, s);
         return e == cudaSuccess ? GPUFFT_SUCCESS : cuda_error(e, "launch pass B (specialised)");
     }
-    if (!P.fb && axis::has_b(P)) return axis::launch_b(P, data, s, fwd, scale, dealias);
     if (fwd)
         pass_b_kernel<T, true><<<P.grid_b, kThreads, P.smem_b, s>>>(prm);
     else
@@ -1117,7 +1153,7 @@ int plan_exec_pass_a_xch(const Plan *P, void *data, void *xch, int nyl, long lon
                                     : launch_pass_a<double>(*P, data, s, forward, &x);
 }
 
-int plan_launches(const Plan *P) { return P ? (P->nx == 1 ? 1 : 2) + ((P->fa ? P->split_a : axis::has_a(*P)) ? 1 : 0) : 0; }
+int plan_launches(const Plan *P) { return P ? (P->nx == 1 ? 1 : 2) + ((P->fa && !P->axis_a ? P->split_a : axis::has_a(*P)) ? 1 : 0) : 0; }
 
 static void describe_axis(std::string &out, const char *name, const AxisPlan &ax) {
     char b[64];
@@ -1160,7 +1196,7 @@ int plan_describe(const Plan *P, char *buf, int len) {
                  P->fb->nt, P->fb->v, P->grid_fb, P->occ_fb, P->fb->smem);
         s += b;
     }
-    axis::form_describe(*P, s, !P->fa, !P->fb);
+    axis::form_describe(*P, s, !P->fa || P->axis_a, !P->fb || P->axis_b);
     if (buf && len > 0) {
         strncpy(buf, s.c_str(), (size_t)len - 1);
         buf[len - 1] = 0;

@@ -49,8 +49,11 @@ struct Plan {
     const void *q_unp = nullptr;    // forward unpack factors
     const void *q_unp_i = nullptr;  // inverse pack factors
     const void *q_rtw = nullptr;  // the row FFT's step-1 twiddles
-    // one-axis-per-launch kernels (axis.cu), made when a pass has no specialised kernel
+    // one-axis-per-launch kernels (axis.cu), made when a pass has no
+    // specialised kernel or they are the faster choice (axis_a, axis_b: they run
+    // although fa or fb names a kernel; the exchange layout still takes fa's)
     axis::Form *axis = nullptr;
+    bool axis_a = false, axis_b = false;
 };
 
 namespace axis {
