@@ -217,6 +217,13 @@ template <typename T> struct ColOut {
     }
 };
 
+// A launch that follows another one of the same transform may start while
+// that one drains (programmatic dependent launch): its tables and barriers are
+// set up meanwhile, and nothing of the field is touched before the first wait
+// here.  A CTA lets the next launch in when it comes to its last tile.
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // Waits for a tile's copy to arrive; false after 2 s, with no copy of either buffer left in flight.
 __device__ __forceinline__ bool arrived(uint64_t *full, int b, uint32_t parity, int *err) {
     constexpr long long kLimit = 2000000000LL;
@@ -307,6 +314,7 @@ __device__ __forceinline__ void cols_body(const ColParams &P, const CUtensorMap 
         fast::cp_async_commit();
     };
     const int grid = gridDim.x;
+    wait_for_previous_launch();
     for (int b = 0; b < P.nbuf; ++b) {
         const int t = blockIdx.x + b * grid;
         if (t < P.ntiles)
@@ -317,6 +325,7 @@ __device__ __forceinline__ void cols_body(const ColParams &P, const CUtensorMap 
     int b = 0;
     uint32_t parity = 0;
     for (int t = blockIdx.x; t < P.ntiles; t += grid) {
+        if (t + grid >= P.ntiles) let_next_launch_start();
         if (tensor && t < P.nfull) {
             if (!arrived(full, b, parity, P.err)) {
                 if (P.nbuf == 2 && t + grid < P.nfull) q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, 2000000000LL);
@@ -409,6 +418,7 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
     // bins k and m - k of one row at a time: `span` adjacent threads take a row
     const int span = min(nt, (half + 31) / 32 * 32), lanes = nt / span, k0 = tid % span, w0 = tid / span;
     const int grid = gridDim.x;
+    wait_for_previous_launch();
     for (int b = 0; b < P.nbuf; ++b) {
         const int t = blockIdx.x + b * grid;
         if (t < P.ntiles)
@@ -420,6 +430,7 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
     int b = 0;
     uint32_t parity = 0;
     for (int t = blockIdx.x; t < P.ntiles; t += grid) {
+        if (t + grid >= P.ntiles) let_next_launch_start();
         if (t < bulk) {
             if (!arrived(full, b, parity, P.err)) {
                 if (P.nbuf == 2 && t + grid < bulk) q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, 2000000000LL);

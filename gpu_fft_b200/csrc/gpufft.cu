@@ -530,7 +530,7 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
 //    against 0.85).  The cluster forms stay for fields of up to 3 MB, where one
 //    launch instead of two is what counts (64^3 0.012 against 0.020; 96^3, 3.6
 //    MB, 0.029 against 0.023; 256^3 0.167 against 0.118; 1024^3 9.68 against
-//    7.51).
+//    7.51).  (Times without the overlap of a transform's launches, axis.cu.)
 //  * x pass: the tensor-copy form stays (512^3 FP32 0.371 against 0.399), as
 //    do short axes and the double-buffered tiles of 128 and 256 points in
 //    FP32 (128 x 512 x 512 0.104 against 0.121); the others go (288^3 0.092
@@ -951,8 +951,9 @@ struct XchLayout {
 };
 
 template <typename T>
-static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, const XchLayout *xch = nullptr) {
-    if ((!P.fa || P.axis_a) && !xch && axis::has_a(P)) return axis::launch_a(P, data, s, fwd);
+static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, const XchLayout *xch = nullptr,
+                         bool chained = false) {
+    if ((!P.fa || P.axis_a) && !xch && axis::has_a(P)) return axis::launch_a(P, data, s, fwd, chained);
     PassAParams prm = P.pa;
     prm.data = data;
     const void *kf = P.fa ? P.fa->kfwd : nullptr, *ki = P.fa ? P.fa->kinv : nullptr;
@@ -1052,9 +1053,10 @@ static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, co
 }
 
 template <typename T>
-static int launch_pass_b(const Plan &P, void *data, cudaStream_t s, bool fwd, double scale = 1.0, int dealias = 0) {
+static int launch_pass_b(const Plan &P, void *data, cudaStream_t s, bool fwd, double scale = 1.0, int dealias = 0,
+                         bool chained = false) {
     if (P.nx == 1) return GPUFFT_SUCCESS;  // a length-1 DFT is the identity
-    if ((!P.fb || P.axis_b) && axis::has_b(P)) return axis::launch_b(P, data, s, fwd, scale, dealias);
+    if ((!P.fb || P.axis_b) && axis::has_b(P)) return axis::launch_b(P, data, s, fwd, scale, dealias, chained);
     PassBParams prm = P.pb;
     prm.data = data;
     prm.scale = scale;
@@ -1103,18 +1105,18 @@ int plan_exec_ex(const Plan *P, void *data, void *stream, bool forward, double s
     if (P->dtype == GPUFFT_FLOAT) {
         if (forward) {
             rc = launch_pass_a<float>(*P, data, s, true);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<float>(*P, data, s, true, scale, dealias);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<float>(*P, data, s, true, scale, dealias, true);
         } else {
             rc = launch_pass_b<float>(*P, data, s, false, scale);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<float>(*P, data, s, false);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<float>(*P, data, s, false, nullptr, P->nx > 1);
         }
     } else {
         if (forward) {
             rc = launch_pass_a<double>(*P, data, s, true);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<double>(*P, data, s, true, scale, dealias);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<double>(*P, data, s, true, scale, dealias, true);
         } else {
             rc = launch_pass_b<double>(*P, data, s, false, scale);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<double>(*P, data, s, false);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<double>(*P, data, s, false, nullptr, P->nx > 1);
         }
     }
     return rc;

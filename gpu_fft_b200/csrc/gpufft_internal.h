@@ -63,8 +63,9 @@ int form_create(Plan &P);
 void form_destroy(Plan &P);
 bool has_a(const Plan &P);
 bool has_b(const Plan &P);
-int launch_a(const Plan &P, void *data, cudaStream_t s, bool fwd);
-int launch_b(const Plan &P, void *data, cudaStream_t s, bool fwd, double scale, int dealias);
+// (chained: the stream's last launch is of the same transform)
+int launch_a(const Plan &P, void *data, cudaStream_t s, bool fwd, bool chained);
+int launch_b(const Plan &P, void *data, cudaStream_t s, bool fwd, double scale, int dealias, bool chained);
 void form_describe(const Plan &P, std::string &out, bool a, bool b);
 }  // namespace axis
 
