@@ -169,6 +169,10 @@ def _stream_handle(stream) -> int:
     import torch
 
     if stream is None:
+        # torch.cuda.current_stream().cuda_stream without the Stream object: 0.2
+        # us a call instead of 3.5, a third of a 32^3 transform's host time
+        if torch.cuda.is_initialized():
+            return int(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
         stream = torch.cuda.current_stream()
     return int(stream.cuda_stream) if hasattr(stream, "cuda_stream") else int(stream)
 

@@ -36,7 +36,9 @@
 
 namespace gpufft {
 
-constexpr int kMaxStages = 24;
+// stages of an axis that fits a tile (up to 16384 points: four of the power of
+// two, then 9s, 5s, ... at least), two such lists in every launch's parameters
+constexpr int kMaxStages = 12;
 constexpr int kThreads = 256;  // threads per CTA for every pass
 
 // One 1D FFT length as its stage list.  Twiddles come from a table of the
