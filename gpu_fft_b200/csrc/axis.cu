@@ -58,7 +58,6 @@ struct Launch {
     int n = 0, w = 0, nt = 0, nbuf = 0, ntiles = 0, grid = 0;
     int copy = 0, boxh = 0, nbox = 0, odd = 0, tile = 0;  // columns: ColParams
     size_t smem = 0, table = 0;  // table: byte offset into Form::dev
-    double bytes = 0;            // of the field
 };
 
 struct Form {
@@ -114,7 +113,6 @@ static int build(Plan &P, Form &F) {
         L.n = n;
         L.w = Width<T>::value;
         L.nt = L.k->nt;
-        L.bytes = (double)nrows * nh * sizeof(V);
         return true;
     };
     // tiles of `groups` groups of gcols columns (ColParams)
@@ -198,12 +196,6 @@ void form_destroy(Plan &P) {
 bool has_a(const Plan &P) { return P.axis && P.axis->has_a; }
 bool has_b(const Plan &P) { return P.axis && P.axis->has_b; }
 
-// chained: the launch before this one in the stream is of the same transform,
-// and this one may start while it drains (griddepcontrol.wait in the kernels).
-// R2C + C2R, us: 100^3 FP32 36.2 -> 26.6, 128^3 47.2 -> 43.0, 200^3 91.6 ->
-// 87.6, 256^3 FP64 312 -> 301, 384 x 360 x 480 FP32 615 -> 605.  Fields above
-// 400 MB gain nothing (500^3 FP32 1185 -> 1195; 420 x 378 x 500, 319 MB, 732
-// both ways) and are launched plainly.
 static cudaError_t launch(const Launch &L, bool fwd, void **args, cudaStream_t s, bool chained) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -211,10 +203,8 @@ static cudaError_t launch(const Launch &L, bool fwd, void **args, cudaStream_t s
     cfg.blockDim = dim3(L.nt);
     cfg.dynamicSmemBytes = L.smem;
     cfg.stream = s;
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = chained && L.bytes <= 400e6 ? 1 : 0;
+    if (chained) attr[cfg.numAttrs++] = dependent_launch();
     return cudaLaunchKernelExC(&cfg, L.fn[fwd], args);
 }
 
@@ -283,8 +273,8 @@ int launch_a(const Plan &P, void *data, cudaStream_t s, bool fwd, bool chained) 
     int rc = GPUFFT_SUCCESS;
     if (fwd) rc = launch_rows(P, F.z, data, s, true, chained);
     if (rc == GPUFFT_SUCCESS)
-        rc = launch_cols(P, F.y, data, s, fwd, nh, P.ny * nh, (int)P.nx, nh, 1.0, 0, fwd || chained);
-    if (!fwd && rc == GPUFFT_SUCCESS) rc = launch_rows(P, F.z, data, s, false, true);
+        rc = launch_cols(P, F.y, data, s, fwd, nh, P.ny * nh, (int)P.nx, nh, 1.0, 0, fwd ? chain_inside(P) : chained);
+    if (!fwd && rc == GPUFFT_SUCCESS) rc = launch_rows(P, F.z, data, s, false, chain_inside(P));
     return rc;
 }
 

@@ -217,13 +217,6 @@ template <typename T> struct ColOut {
     }
 };
 
-// A launch that follows another one of the same transform may start while
-// that one drains (programmatic dependent launch): its tables and barriers are
-// set up meanwhile, and nothing of the field is touched before the first wait
-// here.  A CTA lets the next launch in when it comes to its last tile.
-__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-
 // Waits for a tile's copy to arrive; false after 2 s, with no copy of either buffer left in flight.
 __device__ __forceinline__ bool arrived(uint64_t *full, int b, uint32_t parity, int *err) {
     constexpr long long kLimit = 2000000000LL;

@@ -608,7 +608,9 @@ __device__ __forceinline__ void pass_b_fast_run(const PassBParams &P, unsigned c
     // (the first stage's barrier orders these writes before any twiddle read)
     V *base = reinterpret_cast<V *>(P.data);
     const long long ncols = P.ncols;
+    wait_for_previous_launch();
     for (long long t = first_tile; t < P.ntiles; t += tile_step) {
+        if (t + tile_step >= P.ntiles) let_next_launch_start();
         const long long c0 = t * W;
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = base + c0;
@@ -691,9 +693,11 @@ __global__ void __launch_bounds__(NT, MINB) pass_b_pipe(PassBParams P) {
         cp_async_commit();
     };
     long long t = blockIdx.x;
+    wait_for_previous_launch();
     if (t < P.ntiles) prefetch(t, buf0);
     int k = 0;
     for (; t < P.ntiles; t += gridDim.x, k ^= 1) {
+        if (t + gridDim.x >= P.ntiles) let_next_launch_start();
         V *cur = k ? buf1 : buf0;
         V *nxt = k ? buf0 : buf1;
         const long long tn = t + gridDim.x;
@@ -760,8 +764,10 @@ __global__ void __launch_bounds__(NT, MINB) pass_b_pipe1(PassBParams P) {
         cp_async_commit();
     };
     long long t = blockIdx.x;
+    wait_for_previous_launch();
     if (t < P.ntiles) prefetch(t);
     for (; t < P.ntiles; t += gridDim.x) {
+        if (t + gridDim.x >= P.ntiles) let_next_launch_start();
         cp_async_wait<0>();
         // (the first stage begins with a block barrier: every thread's copies
         // have landed before any thread reads the tile)
@@ -844,6 +850,7 @@ __device__ __forceinline__ void pass_a_fast_run(const PassAParams &P, unsigned c
     for (int q = threadIdx.x; q < M - 1; q += NT) stz[q] = reinterpret_cast<const V *>(P.stz)[q];
     for (int q = threadIdx.x; q < NY - 1; q += NT) sty[q] = reinterpret_cast<const V *>(P.sty)[q];
     __syncthreads();
+    wait_for_previous_launch();
 
     const int cid = first_plane, ncl = plane_step;
     const int rows_per = (NY + K - 1) / K;
@@ -1041,6 +1048,7 @@ __device__ __forceinline__ void pass_a_fast_run(const PassAParams &P, unsigned c
     // while a cluster works on them) runs one of the two phases per launch.
     const bool do_rows = P.phases != 2, do_cols = P.phases != 1;
     for (int plane = cid; plane < P.nx; plane += ncl) {
+        if (plane + ncl >= P.nx) let_next_launch_start();
         V *g = base + (long long)plane * NY * NH;
         if (FWD) {
             if (do_rows) rows(g);

@@ -150,6 +150,15 @@ __device__ __forceinline__ double2 ld_g(const double2 *p) { return __ldcg(p); }
 __device__ __forceinline__ void st_g(float2 *p, float2 v) { __stcg(p, v); }
 __device__ __forceinline__ void st_g(double2 *p, double2 v) { __stcg(p, v); }
 
+// Programmatic dependent launches: a kernel launched as one may start while the
+// launch before it in the stream drains.  It sets its tables (and barriers) up
+// meanwhile and touches nothing of the field before wait_for_previous_launch()
+// -- which returns at once in a plain launch -- has seen that launch complete.
+// let_next_launch_start(), called as a CTA comes to its last tile, lets the
+// next launch in.
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 template <typename T> struct MaxE;
 template <> struct MaxE<float> { static constexpr int value = 32; };
 template <> struct MaxE<double> { static constexpr int value = 16; };

@@ -1024,7 +1024,7 @@ static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, co
         prm.K = P.k_fa;
         prm.phases = 0;
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         cfg.gridDim = dim3(P.grid_fa, 1, 1);
         cfg.blockDim = dim3(P.fa->nt, 1, 1);
         cfg.dynamicSmemBytes = P.fa->smem;
@@ -1035,6 +1035,7 @@ static int launch_pass_a(const Plan &P, void *data, cudaStream_t s, bool fwd, co
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
+        if (chained && P.fa->kind == 0) attr[cfg.numAttrs++] = dependent_launch();
         void *args[] = {&prm};
         const cudaError_t e = cudaLaunchKernelExC(&cfg, fwd ? kf : ki, args);
         return e == cudaSuccess ? GPUFFT_SUCCESS : cuda_error(e, "launch pass A (specialised)");
@@ -1085,7 +1086,15 @@ static int launch_pass_b(const Plan &P, void *data, cudaStream_t s, bool fwd, do
         prm.ntiles = (prm.ncols + P.fb->w - 1) / P.fb->w;
         void *args[] = {&prm};
         const void *k = prm.epi ? (fwd ? P.fb->kfwd_epi : P.fb->kinv_epi) : (fwd ? P.fb->kfwd : P.fb->kinv);
-        const cudaError_t e = cudaLaunchKernel(k, dim3(P.grid_fb), dim3(P.fb->nt), args, P.fb->smem, s);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cfg.gridDim = dim3(P.grid_fb);
+        cfg.blockDim = dim3(P.fb->nt);
+        cfg.dynamicSmemBytes = P.fb->smem;
+        cfg.stream = s;
+        cfg.attrs = attr;
+        if (chained) attr[cfg.numAttrs++] = dependent_launch();
+        const cudaError_t e = cudaLaunchKernelExC(&cfg, k, args);
         return e == cudaSuccess ? GPUFFT_SUCCESS : cuda_error(e, "launch pass B (specialised)");
     }
     if (fwd)
@@ -1105,22 +1114,23 @@ int plan_exec_ex(const Plan *P, void *data, void *stream, bool forward, double s
         return set_error(GPUFFT_ERR_UNSUPPORTED, "Nx = 1 has no x pass to fuse the scale or dealiasing into");
     if (dealias && !forward) return set_error(GPUFFT_ERR_INVALID, "dealiasing is fused into R2C only");
     cudaStream_t s = (cudaStream_t)stream;
+    const bool inside = chain_inside(*P), first = chain_first(*P, s);
     int rc;
     if (P->dtype == GPUFFT_FLOAT) {
         if (forward) {
-            rc = launch_pass_a<float>(*P, data, s, true);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<float>(*P, data, s, true, scale, dealias, true);
+            rc = launch_pass_a<float>(*P, data, s, true, nullptr, first);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<float>(*P, data, s, true, scale, dealias, inside);
         } else {
-            rc = launch_pass_b<float>(*P, data, s, false, scale);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<float>(*P, data, s, false, nullptr, P->nx > 1);
+            rc = launch_pass_b<float>(*P, data, s, false, scale, 0, first);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<float>(*P, data, s, false, nullptr, P->nx > 1 ? inside : first);
         }
     } else {
         if (forward) {
-            rc = launch_pass_a<double>(*P, data, s, true);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<double>(*P, data, s, true, scale, dealias, true);
+            rc = launch_pass_a<double>(*P, data, s, true, nullptr, first);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_b<double>(*P, data, s, true, scale, dealias, inside);
         } else {
-            rc = launch_pass_b<double>(*P, data, s, false, scale);
-            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<double>(*P, data, s, false, nullptr, P->nx > 1);
+            rc = launch_pass_b<double>(*P, data, s, false, scale, 0, first);
+            if (rc == GPUFFT_SUCCESS) rc = launch_pass_a<double>(*P, data, s, false, nullptr, P->nx > 1 ? inside : first);
         }
     }
     return rc;
