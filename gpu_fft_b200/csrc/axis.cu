@@ -151,7 +151,7 @@ static int build(Plan &P, Form &F) {
         L.ntiles = (int)((nrows + L.w - 1) / L.w);
         const int half = m / 2 + 1;
         if (size_launch(L, true, (size_t)((half + m + 1) / 2 * 2) * sizeof(V),
-                        (size_t)((nh * (L.w + 1) + 1) / 2 * 2) * sizeof(V), sms, limit)) {
+                        (size_t)row_tile<V>(m, L.w) * sizeof(V), sms, limit)) {
             L.table = tab.size();
             stage_table<T>(tab, L.n, L.k->r);
             F.unp = tab.size();

@@ -92,6 +92,16 @@ template <typename V> __host__ __device__ constexpr int col_table_bytes(int n) {
     return (n * (int)sizeof(V) + 127) / 128 * 128;
 }
 
+// elements between the rows of a row tile (rows_body), and of a tile buffer
+template <typename V> __host__ __device__ constexpr int row_pitch(int m) {
+    const int nh = m + 1;
+    return nh % 2 ? nh : sizeof(V) == 16 ? nh + 1 : nh % 4 ? nh : nh + 2;  // (FP32: rows 16-byte aligned)
+}
+template <typename V> __host__ __device__ constexpr int row_tile(int m, int w) {
+    const int a = (m + 1) * (w + 1), b = w * row_pitch<V>(m);
+    return ((a > b ? a : b) + 1) / 2 * 2;
+}
+
 // sequences per tile for which a tile row is 128 bytes
 template <typename T> struct Width;
 template <> struct Width<float> { static constexpr int value = 16; };
@@ -103,13 +113,16 @@ enum Lie {
     FIRST,  // the first stage of a column: n * PW + w, or even and odd rows apart (copies 2 and 3)
     ROW     // the first stage of a row: n + w * in_w
 };
+// Where a stage's results go: n * PW + w of the tile, n + w * in_w (the last
+// stage of an inverse row), or out.put (the last stage of a column).
+enum To { IN_PLACE, TO_ROWS, TO_OUT };
 // a thread's part of a tile
 template <typename T> struct Ctx {
     using V = cx_t<T>;
     V *sm;
     const V *tw;
     int w, i0, g;          // this thread's sequence, first butterfly and butterfly step
-    int in_w;              // ROW
+    int in_w;              // ROW, TO_ROWS
     bool apart;            // FIRST: input n at n / 2 * (PW + 2) + (n % 2) * in1 + in0 + w
     int in1, in0;
 };
@@ -127,7 +140,7 @@ __device__ __forceinline__ void load_apart(V (&v)[R], const V *at, int in1, int 
 // One stage in place in shared memory, its results in the layout n * PW + w,
 // or handed to out.put (the last stage of a column).  `freed` runs once every
 // thread has read its inputs.
-template <typename T, class S, bool FWD, int PW, Lie LIE, bool TO_OUT, class Out, class Freed>
+template <typename T, class S, bool FWD, int PW, Lie LIE, To TO, class Out, class Freed>
 __device__ __forceinline__ void stage(const Ctx<T> &c, Out &out, Freed &freed) {
     using V = cx_t<T>;
     constexpr int R = S::r, C = S::c, NB = S::nb, P = S::p;
@@ -150,7 +163,7 @@ __device__ __forceinline__ void stage(const Ctx<T> &c, Out &out, Freed &freed) {
         }
     }
     __syncthreads();
-    if constexpr (TO_OUT) freed();
+    if constexpr (TO == TO_OUT) freed();
 #pragma unroll
     for (int m = 0; m < C; ++m) {
         const int i = c.i0 + m * c.g;
@@ -163,8 +176,12 @@ __device__ __forceinline__ void stage(const Ctx<T> &c, Out &out, Freed &freed) {
                 for (int j = 1; j < R; ++j) v[m][j] = c_tw<FWD>(v[m][j], tw[(j - 1) * P]);
             }
             Dft<R, FWD, V>::run(v[m]);
-            if constexpr (TO_OUT) {
+            if constexpr (TO == TO_OUT) {
                 out.template put<R>(i, NB, v[m]);
+            } else if constexpr (TO == TO_ROWS) {
+                V *o = c.sm + c.w * c.in_w + ip * P * R + k;
+#pragma unroll
+                for (int j = 0; j < R; ++j) o[j * P] = v[m][j];
             } else {
                 V *o = c.sm + (ip * P * R + k) * PW + c.w;
     #pragma unroll
@@ -172,7 +189,7 @@ __device__ __forceinline__ void stage(const Ctx<T> &c, Out &out, Freed &freed) {
             }
         }
     }
-    if constexpr (!TO_OUT) __syncthreads();
+    if constexpr (TO != TO_OUT) __syncthreads();
 }
 
 // The axis of length R1 * R2 * R3 (R3 = 1: two stages) on tiles of W
@@ -339,8 +356,8 @@ __device__ __forceinline__ void cols_body(const ColParams &P, const CUtensorMap 
         const Ctx<T> c{cur, tw, tid % W, tid / W, nt / W, 0, apart, P.odd + 1 - 2 * off, off};
         NoOut none;
         NoFreed nothing;
-        stage<T, typename A::S0, FWD, W, FIRST, false>(c, none, nothing);
-        if constexpr (A::nst == 3) stage<T, typename A::S1, FWD, W, TILE, false>(c, none, nothing);
+        stage<T, typename A::S0, FWD, W, FIRST, IN_PLACE>(c, none, nothing);
+        if constexpr (A::nst == 3) stage<T, typename A::S1, FWD, W, TILE, IN_PLACE>(c, none, nothing);
         ColOut<T> out;
         out.base = valid ? data + (long long)g * P.gstride + col : nullptr;
         out.pitch = P.pitch;
@@ -359,7 +376,7 @@ __device__ __forceinline__ void cols_body(const ColParams &P, const CUtensorMap 
                 fast::cp_async_commit();
         };
         using Last = std::conditional_t<A::nst == 3, typename A::S2, typename A::S1>;
-        stage<T, Last, FWD, W, TILE, true>(c, out, freed);
+        stage<T, Last, FWD, W, TILE, TO_OUT>(c, out, freed);
         if (P.nbuf == 2) {
             b ^= 1;
             parity ^= b == 0;
@@ -370,18 +387,22 @@ __device__ __forceinline__ void cols_body(const ColParams &P, const CUtensorMap 
 }
 
 // Rows.  A tile is W whole rows, one contiguous span of the field, copied in
-// as it is (row w at w * nh: odd for most grids, so that reading W rows at
-// one position is conflict-free); the first stage turns it over to n * PW + w.
+// row after row; the first stage turns it over to n * PW + w.  Rows lie PITCH
+// apart: nh where that keeps W rows' elements at one position out of each
+// other's banks (odd nh: one bulk copy for the tile), else padded (a bulk copy
+// a row).  The inverse's last stage turns the tile back, and bulk stores write
+// it out as it came.
 template <typename T, bool FWD, class A>
 __device__ __forceinline__ void rows_body(const RowParams &P) {
     using V = cx_t<T>;
     constexpr int W = A::W, PW = W + 1, m = A::n, nh = m + 1, half = m / 2 + 1, nt = A::nt;
+    constexpr int PITCH = row_pitch<V>(m), E = (int)sizeof(V);
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x;
     V *unp = reinterpret_cast<V *>(smem_raw);      // half entries
     V *tw = unp + half;                            // m - 1 entries
     V *buf = unp + (half + m + 1) / 2 * 2;
-    const int tile = (nh * PW + 1) / 2 * 2;
+    constexpr int tile = row_tile<V>(m, W);
     uint64_t *full = reinterpret_cast<uint64_t *>(buf + P.nbuf * tile);
     for (int q = tid; q < half; q += nt) unp[q] = reinterpret_cast<const V *>(P.unp)[q];
     for (int q = tid; q < m - 1; q += nt) tw[q] = reinterpret_cast<const V *>(P.tw)[q];
@@ -391,25 +412,36 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
     }
     __syncthreads();
     V *data = reinterpret_cast<V *>(P.data);
-    // a tile is one span: one bulk copy where its ends are 16-byte aligned (whole tiles are, of aligned fields)
-    const int bulk = P.aligned ? P.nrows / W + (sizeof(V) == 16 || P.nrows % W * nh % 2 == 0) : 0;
+    // tiles that go by bulk copies: those whose ends are 16-byte aligned (whole tiles are, of aligned fields)
+    const int bulk = P.aligned ? P.nrows / W + (E == 16 || P.nrows % W * nh % 2 == 0) : 0;
+    // the threads that issue them: one for the tile, or one a row
+    constexpr bool whole = PITCH == nh;
     auto fetch = [&](int t, int b) {
-        const int total = min(W, P.nrows - t * W) * nh;
+        const int rows = min(W, P.nrows - t * W);
         const V *src = data + (long long)t * W * nh;
         V *dst = buf + b * tile;
         if (t < bulk) {
-            if (tid == 0) {
-                q::fence_proxy_async_shared();  // (the buffer's last readers are behind a block barrier)
-                q::mbar_arrive_expect_tx(&full[b], (uint32_t)(total * (int)sizeof(V)));
-                q::bulk_load(dst, src, (uint32_t)(total * (int)sizeof(V)), &full[b]);
+            if (tid < (whole ? 1 : rows)) {
+                if (!FWD) q::bulk_wait_read();       // (this thread's stores from the buffer have read it)
+                q::fence_proxy_async_shared();       // (its last readers are behind a block barrier)
+                if (tid == 0) q::mbar_arrive_expect_tx(&full[b], (uint32_t)(rows * nh * E));
+                q::bulk_load(dst + tid * PITCH, src + tid * nh, (uint32_t)((whole ? rows : 1) * nh * E), &full[b]);
             }
         } else {
-            for (int q = tid; q < total; q += nt) fast::cp_async_elem(dst + q, src + q, true);
+            if (!FWD) {  // (the buffer's last tile may have gone by bulk stores)
+                q::bulk_wait_read();
+                __syncthreads();
+            }
+            for (int q = tid; q < rows * nh; q += nt) {
+                const int w = q / nh;
+                fast::cp_async_elem(dst + q + w * (PITCH - nh), src + q, true);
+            }
         }
         fast::cp_async_commit();
     };
     // bins k and m - k of one row at a time: `span` adjacent threads take a row
-    const int span = min(nt, (half + 31) / 32 * 32), lanes = nt / span, k0 = tid % span, w0 = tid / span;
+    constexpr int span = nt < (half + 31) / 32 * 32 ? nt : (half + 31) / 32 * 32, lanes = nt / span;
+    const int k0 = tid % span, w0 = tid / span;
     const int grid = gridDim.x;
     wait_for_previous_launch();
     for (int b = 0; b < P.nbuf; ++b) {
@@ -426,16 +458,21 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
         if (t + grid >= P.ntiles) let_next_launch_start();
         if (t < bulk) {
             if (!arrived(full, b, parity, P.err)) {
-                if (P.nbuf == 2 && t + grid < bulk) q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, 2000000000LL);
+                if (P.nbuf == 2 && t + grid < bulk && (FWD || t == (int)blockIdx.x))
+                    q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, 2000000000LL);
+                if (!FWD) q::bulk_wait_all();
                 return;
             }
         } else {
-            if (P.nbuf == 2)
+            if (FWD && P.nbuf == 2)
                 fast::cp_async_wait<1>();
             else
                 fast::cp_async_wait<0>();
             __syncthreads();
         }
+        // (the inverse refills the other buffer here, a tile later than it was read: its bulk store has
+        // read it by now)
+        if (!FWD && P.nbuf == 2 && t != (int)blockIdx.x && t + grid < P.ntiles) fetch(t + grid, b ^ 1);
         V *cur = buf + b * tile;
         NoOut none;
         NoFreed nothing;
@@ -448,7 +485,7 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
                 for (int k = k0; k < half; k += span) {
                     const V u = unp[k];
                     for (int w = w0; w < rows; w += lanes) {
-                        V *row = cur + w * nh;
+                        V *row = cur + w * PITCH;
                         V a = row[k], x = row[m - k];
                         if (k == 0) a.y = x.y = (T)0;
                         const V s = V{a.x + x.x, a.y - x.y}, d = V{a.x - x.x, a.y + x.y};
@@ -460,10 +497,11 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
             }
             __syncthreads();
         }
-        const Ctx<T> c{cur, tw, tid % W, tid / W, nt / W, nh, false, 0, 0};
-        stage<T, typename A::S0, FWD, PW, ROW, false>(c, none, nothing);
-        stage<T, typename A::S1, FWD, PW, TILE, false>(c, none, nothing);
-        if constexpr (A::nst == 3) stage<T, typename A::S2, FWD, PW, TILE, false>(c, none, nothing);
+        const Ctx<T> c{cur, tw, tid % W, tid / W, nt / W, PITCH, false, 0, 0};
+        constexpr To last = FWD ? IN_PLACE : TO_ROWS;
+        stage<T, typename A::S0, FWD, PW, ROW, IN_PLACE>(c, none, nothing);
+        stage<T, typename A::S1, FWD, PW, TILE, A::nst == 3 ? IN_PLACE : last>(c, none, nothing);
+        if constexpr (A::nst == 3) stage<T, typename A::S2, FWD, PW, TILE, last>(c, none, nothing);
         if constexpr (FWD) {
             // X[k] = E + O, X[m-k] = conj(E - O), E = (Z[k] + conj Z[m-k]) / 2,
             // O = -i w^k (Z[k] - conj Z[m-k]) / 2; Z[m] = Z[0]
@@ -481,24 +519,27 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
                     }
                 }
             }
+            __syncthreads();
         } else {
-            // the reals, and the two cells of padding as zero
-            const int ospan = min(nt, (nh + 31) / 32 * 32), olanes = nt / ospan, oj = tid % ospan, ow = tid / ospan;
-            if (ow < olanes) {
-                for (int j = oj; j < nh; j += ospan) {
-                    const V *in = cur + j * PW + ow;
-                    V *out = dst + ow * nh + j;
-                    for (int w = ow; w < rows; w += olanes, in += olanes, out += olanes * nh)
-                        st_g(out, j < m ? *in : V{(T)0, (T)0});
-                }
+            // the two cells of padding as zero, then the rows as they lie
+            if (tid < rows) cur[tid * PITCH + m] = V{(T)0, (T)0};
+            if (t < bulk) q::fence_proxy_async_shared();
+            __syncthreads();
+            if (t < bulk) {
+                if (tid < (whole ? 1 : rows))
+                    q::bulk_store(dst + tid * nh, cur + tid * PITCH, (uint32_t)((whole ? rows : 1) * nh * E));
+            } else {
+                for (int q = tid; q < rows * nh; q += nt) st_g(dst + q, cur[q + q / nh * (PITCH - nh)]);
+                __syncthreads();
             }
         }
-        __syncthreads();
-        const int tn = t + P.nbuf * grid;
-        if (tn < P.ntiles)
-            fetch(tn, b);
-        else
-            fast::cp_async_commit();
+        if (FWD || P.nbuf == 1) {
+            const int tn = t + P.nbuf * grid;
+            if (tn < P.ntiles)
+                fetch(tn, b);
+            else
+                fast::cp_async_commit();
+        }
         if (P.nbuf == 2) {
             b ^= 1;
             parity ^= b == 0;
@@ -506,6 +547,7 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
             parity ^= 1;
         }
     }
+    if (!FWD) q::bulk_wait_all();
 }
 
 // Threads and CTAs per SM of a length R1 * R2 (R1 >= R2).  The second stage
