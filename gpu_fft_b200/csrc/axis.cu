@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <new>
 #include <vector>
 
 #include "../../include/gpufft_b200.h"
@@ -182,8 +183,11 @@ static int build(Plan &P, Form &F) {
 
 int form_create(Plan &P) {
     if (P.axis) return GPUFFT_SUCCESS;
-    P.axis = new Form();
-    return P.dtype == GPUFFT_FLOAT ? build<float>(P, *P.axis) : build<double>(P, *P.axis);
+    P.axis = new (std::nothrow) Form();
+    if (!P.axis) return set_error(GPUFFT_ERR_OOM, "host allocation failed");
+    const int rc = P.dtype == GPUFFT_FLOAT ? build<float>(P, *P.axis) : build<double>(P, *P.axis);
+    if (rc != GPUFFT_SUCCESS) P.axis->has_a = P.axis->has_b = false;
+    return rc;
 }
 
 void form_destroy(Plan &P) {

@@ -525,11 +525,11 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
 // one-axis-per-launch kernels over the registered ones where they measured
 // faster (ms per launch or pair of launches, forward + inverse):
 //  * Pass A: the queue form stays at 512^2 planes (512^3 FP32 0.72 against
-//    0.86, FP64 1.50 against 1.58), at 512 x 128 in FP32 and 360 x 240 in
-//    FP64, but goes at 512 x 128 in FP64 and 360 x 240 in FP32 (R2C + C2R in
-//    a row until the 1000 W cap holds the clock, where the form that crosses
-//    HBM less often gains: 1.283 against 1.319, 1.257 against 1.274, but 2.640
-//    against 2.504, 0.642 against 0.630).  The cluster forms stay for fields
+//    0.80, FP64 1.50 against 1.56) and at 512 x 128 in FP32, but goes at 512 x
+//    128 in FP64 and at 360 x 240 (R2C + C2R in a row until the 1000 W cap holds
+//    the clock, where the form that crosses HBM less often gains: 1.297 against
+//    1.320, but 2.646 against 2.469, 0.650 against 0.615 and FP64 1.285 against
+//    1.255).  The cluster forms stay for fields
 //    of up to 3 MB, where one launch instead of two is what counts (64^3 0.012
 //    against 0.020; 96^3, 3.6 MB, 0.029 against 0.023; 256^3 0.167 against
 //    0.118; 1024^3 9.68 against 7.51).  (Single launches without the overlap
@@ -543,7 +543,7 @@ static int prefer_axis(Plan &P, bool pick_a, bool pick_b) {
     const double bytes = (double)P.nx * P.ny * (P.nz / 2 + 1) * (P.dtype == GPUFFT_FLOAT ? 8 : 16);
     bool a = false, b = false;
     if (pick_a && P.fa)
-        a = P.fa->kind == 2 ? P.fa->m == (P.dtype == GPUFFT_FLOAT ? 240 : 128) : bytes > 3e6;
+        a = P.fa->kind == 2 ? P.fa->m != 256 && !(P.fa->m == 128 && P.dtype == GPUFFT_FLOAT) : bytes > 3e6;
     if (pick_b && P.fb && !P.tc_split)
         b = P.fb->kind != 3 && P.nx >= 96 &&
             !(P.dtype == GPUFFT_FLOAT && P.fb->kind == 1 && (P.nx == 128 || P.nx == 256));
@@ -1347,7 +1347,8 @@ extern "C" int gpufft_plan_check(gpufft_plan plan) {
     if (e != cudaSuccess) return cuda_error(e, "read the plan's device flags");
     if (tc || qe)
         return set_error(GPUFFT_ERR_CUDA, "a bounded device-side wait of this plan's kernels ran out (%s%s%s)",
-                         qe ? "queue Pass A" : "", qe && tc ? ", " : "", tc ? "tensor-core x pass" : "");
+                         qe ? "queue Pass A" : "", qe && tc ? ", " : "",
+                         tc ? "tensor-core x pass or axis kernels" : "");
     return GPUFFT_SUCCESS;
 }
 
