@@ -223,11 +223,14 @@ template <typename T> struct ColOut {
         if (!epi) {
 #pragma unroll
             for (int j = 0; j < R; ++j) st_g(o + (size_t)j * step, v[j]);
+        } else if (!nx) {
+#pragma unroll
+            for (int j = 0; j < R; ++j) st_g(o + (size_t)j * step, V{v[j].x * scale, v[j].y * scale});
         } else {
 #pragma unroll
             for (int j = 0; j < R; ++j) {
                 const int kx = i + j * nb;
-                const bool zero = nx && (drop || 3 * min(kx, nx - kx) > nx);
+                const bool zero = (drop || 3 * min(kx, nx - kx) > nx);
                 st_g(o + (size_t)j * step, zero ? V{(T)0, (T)0} : V{v[j].x * scale, v[j].y * scale});
             }
         }
