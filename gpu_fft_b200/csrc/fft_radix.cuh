@@ -4,7 +4,9 @@
 // with s = -1 (FWD) or +1 (inverse), unscaled — the convention of the
 // transforms GPU_FFT calls (cuFFT FORWARD/INVERSE, FFT_R2C.cu:69, FFT_C2R.cu:45).
 // Radix 2, 4, 8, 9 and 16 are hand-factored (4 = 2x2, 8 = 2x4, 9 = 3x3,
-// 16 = 4x4 with constant twiddles); odd primes 3..13 use the symmetric pair form
+// 16 = 4x4 with constant twiddles); other composites up to 32 are prime-factor
+// (DftPfa) or Cooley-Tukey (DftCt) compositions of these; odd primes 3..13 use
+// the symmetric pair form
 //   y[k] = x0 + sum_{j<=(R-1)/2} cos(2pi jk/R)(x_j + x_{R-j})  -/+  i sin(2pi jk/R)(x_j - x_{R-j}).
 // The trigonometric constants are the mathematical values written out to
 // 25 significant digits and rounded by the compiler to the storage type.
