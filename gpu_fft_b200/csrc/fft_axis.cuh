@@ -424,8 +424,11 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
         const V *src = data + (long long)t * W * nh;
         V *dst = buf + b * tile;
         if (t < bulk) {
+            // Every thread that stored from the buffer waits until its stores have read it, also those
+            // that have no row of this tile (the last one): the stages write over the whole buffer, behind
+            // the block barrier that follows the pack.
+            if (!FWD && tid < (whole ? 1 : W)) q::bulk_wait_read();
             if (tid < (whole ? 1 : rows)) {
-                if (!FWD) q::bulk_wait_read();       // (this thread's stores from the buffer have read it)
                 q::fence_proxy_async_shared();       // (its last readers are behind a block barrier)
                 if (tid == 0) q::mbar_arrive_expect_tx(&full[b], (uint32_t)(rows * nh * E));
                 q::bulk_load(dst + tid * PITCH, src + tid * nh, (uint32_t)((whole ? rows : 1) * nh * E), &full[b]);

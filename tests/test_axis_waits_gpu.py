@@ -1,0 +1,43 @@
+"""GPU tests of what the one-axis-per-launch kernels (fft_axis.cuh) wait for:
+their own copies and the launches around them."""
+import pytest
+
+from test_axis_gpu import _make, _noalloc, _rel, _tol
+
+pytestmark = pytest.mark.gpu
+
+
+def _launch(describe, name):
+    """The numbers of one axis launch in Plan.describe(): {"grid": ..., "nbuf": ...}."""
+    part = describe.split(name + "{")[1].split("}")[0]
+    return {k: int(v) for k, v in (w.split("=") for w in part.split()) if v.isdigit()}
+
+
+# FP64 rows of even Nh and FP32 rows of Nh a multiple of 4 lie padded in shared memory and are stored one by one;
+# 54675 and 15015 rows leave a last tile of a few rows, which takes the place of a whole one
+@pytest.mark.parametrize("grid, dt, nbuf", [((225, 243, 126), "float", 2), ((225, 243, 126), "double", 2),
+                                            ((105, 143, 910), "float", 1), ((105, 143, 882), "double", 1)], ids=str)
+def test_inverse_rows_refilled_by_a_partial_last_tile(cuda, grid, dt, nbuf, monkeypatch):
+    import torch
+    import gpu_fft_b200 as g
+
+    monkeypatch.setenv("GPUFFT_GENERIC_ONLY", "1")
+    p = g.Plan(*grid, dt)
+    w = 16 if dt == "float" else 8
+    z = _launch(p.describe(), "axisZ")
+    rows = grid[0] * grid[1]
+    assert z["nbuf"] == nbuf
+    assert rows % w and -(-rows // w) > z["nbuf"] * z["grid"]  # the last tile refills a buffer
+    s = _make(grid, dt, 12)
+    want = s.clone()
+    _noalloc(g, grid, dt, False, want)
+    nz = grid[2]
+    first = None
+    for _ in range(8):
+        a = s.clone()
+        p.c2r(a)
+        if first is None:
+            assert _rel(a[..., :nz], want[..., :nz]) < _tol(grid, dt)
+            first = a
+        assert torch.equal(a, first)
+    p.check()
