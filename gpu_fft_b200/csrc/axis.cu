@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <new>
 #include <vector>
 
@@ -66,6 +67,8 @@ struct Form {
     size_t unp = 0;  // byte offset of the rows' unpack factors, then the pack factors (RowParams)
     Launch x, y, z;
     bool has_a = false, has_b = false;
+    long long wait_ns = 2000000000LL;  // limit of the wait for a tile's copy: 2 s, far above any launch's length
+    int missing_rows = 0, missing_cols = 0;  // RowParams, ColParams::missing
 };
 
 // Shared memory and grid of a launch; false where one tile does not fit.
@@ -185,6 +188,15 @@ int form_create(Plan &P) {
     if (P.axis) return GPUFFT_SUCCESS;
     P.axis = new (std::nothrow) Form();
     if (!P.axis) return set_error(GPUFFT_ERR_OOM, "host allocation failed");
+    // test hooks of the bounded wait: with GPUFFT_AXIS_UNREACHABLE at plan creation the row tiles (1), the column
+    // tiles (2) or both (3) wait for 16 bytes more than their copies bring, so the wait runs out, after
+    // GPUFFT_AXIS_WAIT_MS, and gpufft_plan_check reports it
+    if (const char *ev = std::getenv("GPUFFT_AXIS_UNREACHABLE")) {
+        const int which = std::atoi(ev);
+        P.axis->missing_rows = which & 1 ? 16 : 0;
+        P.axis->missing_cols = which & 2 ? 16 : 0;
+    }
+    if (const char *ev = std::getenv("GPUFFT_AXIS_WAIT_MS")) P.axis->wait_ns = 1000000LL * std::max(1, std::atoi(ev));
     const int rc = P.dtype == GPUFFT_FLOAT ? build<float>(P, *P.axis) : build<double>(P, *P.axis);
     if (rc != GPUFFT_SUCCESS) P.axis->has_a = P.axis->has_b = false;
     return rc;
@@ -235,6 +247,8 @@ static int launch_cols(const Plan &P, const Launch &L, void *data, cudaStream_t 
     c.tile = L.tile;
     c.gpar = L.copy == 2 ? (int)(gstride % 2) : 0;
     c.err = P.pb.err;
+    c.wait_ns = P.axis->wait_ns;
+    c.missing = P.axis->missing_cols;
     if ((uintptr_t)data % 16) c.copy = 0;
     CUtensorMap tm{};
     if (c.copy == 1) {
@@ -266,6 +280,9 @@ static int launch_rows(const Plan &P, const Launch &L, void *data, cudaStream_t 
     p.aligned = (uintptr_t)data % 16 == 0;
     p.ntiles = L.ntiles;
     p.nbuf = L.nbuf;
+    p.err = P.pb.err;
+    p.wait_ns = P.axis->wait_ns;
+    p.missing = P.axis->missing_rows;
     void *args[] = {&p};
     const cudaError_t e = launch(L, fwd, args, s, chained);
     return e == cudaSuccess ? GPUFFT_SUCCESS : set_error(GPUFFT_ERR_CUDA, "launch axis rows: %s", cudaGetErrorString(e));

@@ -71,7 +71,9 @@ struct ColParams {
     int gpar;  // copy 2: row r of group g is off by 8 bytes where r + gpar * g is odd
     int boxh, nbox;
     int odd;   // copies 2 and 3: where the odd rows of a tile start
-    int *err;  // raised when a copy has not arrived within 2 s (or null)
+    int *err;           // raised when a tile's copy has not arrived within wait_ns
+    long long wait_ns;
+    int missing;        // bytes expected of a tile's copy beyond those it brings: 0 (a test of the limit: more)
     // x-pass epilogue (PassBParams), on when epi is set: scale, and the 2/3-rule mask of column ky * nh + kz
     int epi, dealias, ny, nh, nz;
     double scale;
@@ -85,7 +87,9 @@ struct RowParams {
     int nrows;
     int ntiles, nbuf;
     int aligned;  // data 16-byte aligned
-    int *err;     // as in ColParams
+    int *err;     // these as in ColParams
+    long long wait_ns;
+    int missing;
 };
 
 template <typename V> __host__ __device__ constexpr int col_table_bytes(int n) {
@@ -237,12 +241,14 @@ template <typename T> struct ColOut {
     }
 };
 
-// Waits for a tile's copy to arrive; false after 2 s, with no copy of either buffer left in flight.
-__device__ __forceinline__ bool arrived(uint64_t *full, int b, uint32_t parity, int *err) {
-    constexpr long long kLimit = 2000000000LL;
-    if (q::mbar_wait(&full[b], parity, kLimit)) return true;
-    q::mbar_wait(&full[b], parity, kLimit);
-    if (err) atomicExch(err, 1);
+// Waits for a tile's copy to arrive.  False once the limit has passed: the flag is raised, and the copy has been
+// given the same time again, so that the CTA, which ends now, leaves none in flight into its shared memory unless
+// it takes more than twice the limit.  (The other buffer's copy is the caller's to wait for.)
+template <class Params>
+__device__ __forceinline__ bool arrived(const Params &P, uint64_t *full, int b, uint32_t parity) {
+    if (q::mbar_wait(&full[b], parity, P.wait_ns)) return true;
+    atomicExch(P.err, 1);
+    q::mbar_wait(&full[b], parity, P.wait_ns);
     return false;
 }
 
@@ -289,11 +295,12 @@ __device__ __forceinline__ void cols_body(const ColParams &P, const CUtensorMap 
                 column(t, 0, g, c);
                 q::fence_proxy_async_shared();  // (the buffer's last readers are behind a block barrier)
                 if (P.copy == 1) {
-                    q::mbar_arrive_expect_tx(&full[b], (uint32_t)(P.nbox * P.boxh * W * (int)sizeof(V)));
+                    q::mbar_arrive_expect_tx(&full[b], (uint32_t)(P.nbox * P.boxh * W * (int)sizeof(V) + P.missing));
                     for (int x = 0; x < P.nbox; ++x)
                         q::tensor_load_2d(dst + x * P.boxh * W, &tm, c * E8, g * n + x * P.boxh, &full[b]);
                 } else {
-                    q::mbar_arrive_expect_tx(&full[b], (uint32_t)(2 * P.nbox * P.boxh * (W + 2) * (int)sizeof(V)));
+                    q::mbar_arrive_expect_tx(&full[b],
+                                             (uint32_t)(2 * P.nbox * P.boxh * (W + 2) * (int)sizeof(V) + P.missing));
                     for (int x = 0; x < P.nbox; ++x) {
                         const int at = x * P.boxh * (W + 2), line = g * (n / 2) + x * P.boxh;
                         q::tensor_load_2d(dst + at, &tm, c, line, &full[b]);
@@ -340,8 +347,8 @@ __device__ __forceinline__ void cols_body(const ColParams &P, const CUtensorMap 
     for (int t = blockIdx.x; t < P.ntiles; t += grid) {
         if (t + grid >= P.ntiles) let_next_launch_start();
         if (tensor && t < P.nfull) {
-            if (!arrived(full, b, parity, P.err)) {
-                if (P.nbuf == 2 && t + grid < P.nfull) q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, 2000000000LL);
+            if (!arrived(P, full, b, parity)) {
+                if (P.nbuf == 2 && t + grid < P.nfull) q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, P.wait_ns);
                 return;
             }
         } else {
@@ -430,7 +437,7 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
             if (!FWD && tid < (whole ? 1 : W)) q::bulk_wait_read();
             if (tid < (whole ? 1 : rows)) {
                 q::fence_proxy_async_shared();       // (its last readers are behind a block barrier)
-                if (tid == 0) q::mbar_arrive_expect_tx(&full[b], (uint32_t)(rows * nh * E));
+                if (tid == 0) q::mbar_arrive_expect_tx(&full[b], (uint32_t)(rows * nh * E + P.missing));
                 q::bulk_load(dst + tid * PITCH, src + tid * nh, (uint32_t)((whole ? rows : 1) * nh * E), &full[b]);
             }
         } else {
@@ -463,9 +470,9 @@ __device__ __forceinline__ void rows_body(const RowParams &P) {
     for (int t = blockIdx.x; t < P.ntiles; t += grid) {
         if (t + grid >= P.ntiles) let_next_launch_start();
         if (t < bulk) {
-            if (!arrived(full, b, parity, P.err)) {
+            if (!arrived(P, full, b, parity)) {
                 if (P.nbuf == 2 && t + grid < bulk && (FWD || t == (int)blockIdx.x))
-                    q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, 2000000000LL);
+                    q::mbar_wait(&full[b ^ 1], parity ^ (uint32_t)b, P.wait_ns);
                 if (!FWD) q::bulk_wait_all();
                 return;
             }

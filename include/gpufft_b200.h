@@ -93,9 +93,9 @@ int gpufft_plan_create(gpufft_plan *plan, int64_t nx, int64_t ny, int64_t nz, in
 int gpufft_plan_destroy(gpufft_plan plan);
 /* Reads the plan's device-side error flags (synchronous): GPUFFT_ERR_CUDA if
  * a bounded wait inside one of its kernels ran out since the plan was made
- * (the queue-scheduled Pass A waiting for a plane, or the tensor-core x pass
- * waiting for its MMAs; the results of that call are wrong and the plan
- * should be destroyed), else GPUFFT_SUCCESS.  No reference counterpart. */
+ * (the queue-scheduled Pass A waiting for a plane, the tensor-core x pass
+ * waiting for its MMAs, or a one-axis kernel waiting for a tile's copy; the
+ * results of that call are wrong and the plan should be destroyed), else GPUFFT_SUCCESS.  No reference counterpart. */
 int gpufft_plan_check(gpufft_plan plan);
 int gpufft_exec_r2c(gpufft_plan plan, void *data, void *stream);
 int gpufft_exec_c2r(gpufft_plan plan, void *data, void *stream);

@@ -41,3 +41,40 @@ def test_inverse_rows_refilled_by_a_partial_last_tile(cuda, grid, dt, nbuf, monk
             first = a
         assert torch.equal(a, first)
     p.check()
+
+
+@pytest.mark.parametrize("dt", ["float", "double"])
+@pytest.mark.parametrize("which", [1, 2], ids=["rows", "columns"])
+def test_axis_wait_runs_out_and_reports(cuda, which, dt, monkeypatch):
+    """The copies of the row or the column tiles are waited for 16 bytes too
+    long, with a 20 ms limit: the launches end, plan_check reports it, and the
+    device stays usable."""
+    import time
+
+    import torch
+    import gpu_fft_b200 as g
+
+    grid = (32, 100, 100)
+    monkeypatch.setenv("GPUFFT_GENERIC_ONLY", "1")
+    f = _make(grid, dt, 13)
+    for forward in (True, False):
+        monkeypatch.setenv("GPUFFT_AXIS_UNREACHABLE", str(which))
+        monkeypatch.setenv("GPUFFT_AXIS_WAIT_MS", "20")
+        p = g.Plan(*grid, dt)
+        monkeypatch.delenv("GPUFFT_AXIS_UNREACHABLE")
+        monkeypatch.delenv("GPUFFT_AXIS_WAIT_MS")
+        a = f.clone()
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        (p.r2c if forward else p.c2r)(a)
+        torch.cuda.synchronize()
+        assert time.perf_counter() - t0 < 1.0
+        with pytest.raises(g.GpuFFTError, match="ERR_CUDA"):
+            p.check()
+        p.close()
+    q = g.Plan(*grid, dt)
+    a, want = f.clone(), f.clone()
+    q.r2c(a)
+    _noalloc(g, grid, dt, True, want)
+    assert _rel(a, want) < _tol(grid, dt)
+    q.check()
