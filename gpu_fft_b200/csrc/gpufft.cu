@@ -919,7 +919,6 @@ int plan_adopt(Plan *P, const Plan *Q) {
     if (!P || !Q) return set_error(GPUFFT_ERR_NOT_INIT, "no plan");
     if (P->nx != Q->nx || P->ny != Q->ny || P->nz != Q->nz || P->dtype != Q->dtype || P->tc_split != Q->tc_split)
         return set_error(GPUFFT_ERR_INVALID, "plan_adopt: the plans differ in grid or form");
-    if (Q->idx_a < 0 && Q->idx_b < 0) return GPUFFT_SUCCESS;  // generic kernels: nothing to copy
     P->kfix = Q->kfix;
     int rc = setup_fast(*P, Q->idx_a, Q->idx_b);
     if (rc == GPUFFT_SUCCESS && (Q->axis_a || Q->axis_b)) rc = axis::form_create(*P);

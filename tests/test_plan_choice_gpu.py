@@ -1,0 +1,42 @@
+"""GPU tests of which kernels a plan runs."""
+import ctypes
+
+import pytest
+
+from test_axis_gpu import _make
+
+pytestmark = pytest.mark.gpu
+
+
+def _wisdom(g, tmp_path, grid, a, b):
+    """Plans of the grid (FP32) made from now on are tuned to candidates a and b."""
+    import torch
+
+    dev = torch.cuda.get_device_name(0).replace(" ", "_")
+    major, minor = torch.cuda.get_device_capability(0)
+    path = tmp_path / "w.txt"
+    path.write_text(f"{dev}_sm{major * 10 + minor} 0 {grid[0]} {grid[1]} {grid[2]} {a} {b} 0\n")
+    g.wisdom_load(str(path))
+
+
+def test_a_plan_adopts_the_choice_of_no_registered_kernel(cuda, tmp_path):
+    """A batch tunes one plan of each grid and the others adopt its choice, also
+    where that is the one-axis kernels for both passes (candidates -1, -1)."""
+    import torch
+    import gpu_fft_b200 as g
+
+    grid = (24, 512, 256)  # (512 x 128 planes: the queue form by default)
+    p = g.Plan(*grid, "float")
+    assert "fastA{kind=2 " in p.describe()
+    _wisdom(g, tmp_path, grid, -1, -1)
+    q = g.Plan(*grid, "float")
+    assert "tuned=1 candA=-1 candB=-1" in q.describe() and "fastA" not in q.describe()
+    adopt = g.load_library()["_ZN6gpufft10plan_adoptEPNS_4PlanEPKS0_"]  # gpufft::plan_adopt(Plan *, const Plan *)
+    adopt.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+    assert adopt(p.handle, q.handle) == 0
+    assert p.describe() == q.describe()
+    a = _make(grid, "float", 5)
+    b = a.clone()
+    p.r2c(a)
+    q.r2c(b)
+    assert torch.equal(a, b)
