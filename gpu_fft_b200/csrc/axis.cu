@@ -59,14 +59,20 @@ struct Launch {
     const Kernels *k = nullptr;
     int n = 0, w = 0, nt = 0, nbuf = 0, ntiles = 0, grid = 0;
     int copy = 0, boxh = 0, nbox = 0, odd = 0, tile = 0;  // columns: ColParams
-    size_t smem = 0, table = 0;  // table: byte offset into Form::dev
+    size_t smem = 0, table = 0;  // table: byte offset into the part's tables
+};
+
+// the launches of one pass, its tables on the device
+struct Part {
+    bool made = false, has = false;  // made: form_create has been here; has: these lengths have kernels
+    void *dev = nullptr;
+    size_t bytes = 0;
 };
 
 struct Form {
-    void *dev = nullptr;
+    Part a, b;       // Pass A (z and y), x pass: each made when a plan first needs it
     size_t unp = 0;  // byte offset of the rows' unpack factors, then the pack factors (RowParams)
     Launch x, y, z;
-    bool has_a = false, has_b = false;
     long long wait_ns = 2000000000LL;  // limit of the wait for a tile's copy: 2 s, far above any launch's length
     int missing_rows = 0, missing_cols = 0;  // RowParams, ColParams::missing
 };
@@ -99,7 +105,7 @@ static bool size_launch(Launch &L, bool rows, size_t fixed, size_t tile, int sms
 }
 
 template <typename T>
-static int build(Plan &P, Form &F) {
+static int build(Plan &P, Form &F, Part &part) {
     using V = cx_t<T>;
     const int nx = (int)P.nx, ny = (int)P.ny, m = (int)(P.nz / 2), nh = m + 1;
     int sms = 1, limit = 0;
@@ -149,8 +155,10 @@ static int build(Plan &P, Form &F) {
         stage_table<T>(tab, L.n, L.k->r);
         return true;
     };
-    if (xcols < most) F.has_b = columns(F.x, nx, 1, (int)xcols, xcols);
-    if (ycols < most && nrows < most && columns(F.y, ny, nx, nh, nh) && kernels(F.z, m, false)) {
+    bool has = false;
+    if (&part == &F.b)
+        has = xcols < most && columns(F.x, nx, 1, (int)xcols, xcols);
+    else if (ycols < most && nrows < most && columns(F.y, ny, nx, nh, nh) && kernels(F.z, m, false)) {
         Launch &L = F.z;
         L.ntiles = (int)((nrows + L.w - 1) / L.w);
         const int half = m / 2 + 1;
@@ -170,23 +178,29 @@ static int build(Plan &P, Form &F) {
                 u[2 * (half + k)] = (T)(-sn);
                 u[2 * (half + k) + 1] = (T)c;
             }
-            F.has_a = true;
+            has = true;
         }
     }
-    if (!F.has_a && !F.has_b) return GPUFFT_SUCCESS;
-    cudaError_t e = cudaMalloc(&F.dev, tab.size());
+    if (!has) return GPUFFT_SUCCESS;
+    cudaError_t e = cudaMalloc(&part.dev, tab.size());
     if (e != cudaSuccess) {
-        F.dev = nullptr;
+        part.dev = nullptr;
         return set_error(GPUFFT_ERR_OOM, "cudaMalloc axis tables: %s", cudaGetErrorString(e));
     }
-    e = cudaMemcpy(F.dev, tab.data(), tab.size(), cudaMemcpyHostToDevice);
-    return e == cudaSuccess ? GPUFFT_SUCCESS
-                            : set_error(GPUFFT_ERR_CUDA, "upload axis tables: %s", cudaGetErrorString(e));
+    e = cudaMemcpy(part.dev, tab.data(), tab.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return set_error(GPUFFT_ERR_CUDA, "upload axis tables: %s", cudaGetErrorString(e));
+    part.bytes = tab.size();
+    part.has = true;
+    return GPUFFT_SUCCESS;
 }
 
-int form_create(Plan &P) {
-    if (P.axis) return GPUFFT_SUCCESS;
-    P.axis = new (std::nothrow) Form();
+int form_create(Plan &P, bool a, bool b) {
+    if (P.axis) {
+        a = a && !P.axis->a.made;
+        b = b && !P.axis->b.made;
+    }
+    if (!a && !b) return GPUFFT_SUCCESS;
+    if (!P.axis) P.axis = new (std::nothrow) Form();
     if (!P.axis) return set_error(GPUFFT_ERR_OOM, "host allocation failed");
     // test hooks of the bounded wait: with GPUFFT_AXIS_UNREACHABLE at plan creation the row tiles (1), the column
     // tiles (2) or both (3) wait for 16 bytes more than their copies bring, so the wait runs out, after
@@ -197,20 +211,25 @@ int form_create(Plan &P) {
         P.axis->missing_cols = which & 2 ? 16 : 0;
     }
     if (const char *ev = std::getenv("GPUFFT_AXIS_WAIT_MS")) P.axis->wait_ns = 1000000LL * std::max(1, std::atoi(ev));
-    const int rc = P.dtype == GPUFFT_FLOAT ? build<float>(P, *P.axis) : build<double>(P, *P.axis);
-    if (rc != GPUFFT_SUCCESS) P.axis->has_a = P.axis->has_b = false;
+    int rc = GPUFFT_SUCCESS;
+    for (Part *part : {a ? &P.axis->a : nullptr, b ? &P.axis->b : nullptr}) {
+        if (!part || rc != GPUFFT_SUCCESS) continue;
+        part->made = true;
+        rc = P.dtype == GPUFFT_FLOAT ? build<float>(P, *P.axis, *part) : build<double>(P, *P.axis, *part);
+    }
     return rc;
 }
 
 void form_destroy(Plan &P) {
     if (!P.axis) return;
-    if (P.axis->dev) cudaFree(P.axis->dev);
+    for (Part *part : {&P.axis->a, &P.axis->b})
+        if (part->dev) cudaFree(part->dev);
     delete P.axis;
     P.axis = nullptr;
 }
 
-bool has_a(const Plan &P) { return P.axis && P.axis->has_a; }
-bool has_b(const Plan &P) { return P.axis && P.axis->has_b; }
+bool has_a(const Plan &P) { return P.axis && P.axis->a.has; }
+bool has_b(const Plan &P) { return P.axis && P.axis->b.has; }
 
 static cudaError_t launch(const Launch &L, bool fwd, void **args, cudaStream_t s, bool chained) {
     cudaLaunchConfig_t cfg = {};
@@ -224,11 +243,11 @@ static cudaError_t launch(const Launch &L, bool fwd, void **args, cudaStream_t s
     return cudaLaunchKernelExC(&cfg, L.fn[fwd], args);
 }
 
-static int launch_cols(const Plan &P, const Launch &L, void *data, cudaStream_t s, bool fwd, long long pitch,
+static int launch_cols(const Plan &P, const Part &part, const Launch &L, void *data, cudaStream_t s, bool fwd, long long pitch,
                        long long gstride, int groups, int gcols, double scale, int dealias, bool chained) {
     ColParams c{};
     c.data = data;
-    c.tw = (const char *)P.axis->dev + L.table;
+    c.tw = (const char *)part.dev + L.table;
     c.pitch = pitch;
     c.gstride = gstride;
     c.gcols = gcols;
@@ -273,9 +292,9 @@ static int launch_rows(const Plan &P, const Launch &L, void *data, cudaStream_t 
     const int m = (int)(P.nz / 2);
     RowParams p{};
     p.data = data;
-    p.tw = (const char *)P.axis->dev + L.table;
+    p.tw = (const char *)P.axis->a.dev + L.table;
     const size_t vs = P.dtype == GPUFFT_FLOAT ? sizeof(float2) : sizeof(double2);
-    p.unp = (const char *)P.axis->dev + P.axis->unp + (fwd ? 0 : (size_t)(m / 2 + 1) * vs);
+    p.unp = (const char *)P.axis->a.dev + P.axis->unp + (fwd ? 0 : (size_t)(m / 2 + 1) * vs);
     p.nrows = (int)(P.nx * P.ny);
     p.aligned = (uintptr_t)data % 16 == 0;
     p.ntiles = L.ntiles;
@@ -294,14 +313,14 @@ int launch_a(const Plan &P, void *data, cudaStream_t s, bool fwd, bool chained) 
     int rc = GPUFFT_SUCCESS;
     if (fwd) rc = launch_rows(P, F.z, data, s, true, chained);
     if (rc == GPUFFT_SUCCESS)
-        rc = launch_cols(P, F.y, data, s, fwd, nh, P.ny * nh, (int)P.nx, nh, 1.0, 0, fwd ? chain_inside(P) : chained);
+        rc = launch_cols(P, F.a, F.y, data, s, fwd, nh, P.ny * nh, (int)P.nx, nh, 1.0, 0, fwd ? chain_inside(P) : chained);
     if (!fwd && rc == GPUFFT_SUCCESS) rc = launch_rows(P, F.z, data, s, false, chain_inside(P));
     return rc;
 }
 
 int launch_b(const Plan &P, void *data, cudaStream_t s, bool fwd, double scale, int dealias, bool chained) {
     const int ncols = (int)(P.ny * (P.nz / 2 + 1));
-    return launch_cols(P, P.axis->x, data, s, fwd, ncols, 0, 1, ncols, scale, dealias, chained);
+    return launch_cols(P, P.axis->b, P.axis->x, data, s, fwd, ncols, 0, 1, ncols, scale, dealias, chained);
 }
 
 static void describe(std::string &out, const char *name, const Launch &L) {
@@ -317,6 +336,7 @@ void form_describe(const Plan &P, std::string &out, bool a, bool b) {
         describe(out, "axisY", P.axis->y);
     }
     if (b && has_b(P)) describe(out, "axisX", P.axis->x);
+    if (has_a(P) || has_b(P)) out += " axisTables=" + std::to_string(P.axis->a.bytes + P.axis->b.bytes);
 }
 
 }  // namespace axis

@@ -155,7 +155,7 @@ static int dist_setup(DistPlan *D, int64_t nx, int64_t ny, int64_t nz, int dtype
     D->cs = dtype == GPUFFT_FLOAT ? 8 : 16;
     D->chunk = (size_t)D->nxl * D->nyl * D->nh * D->cs;
     cudaGetDevice(&D->device);
-    int rc = plan_create(&D->pa, D->nxl, ny, nz, dtype, 0);
+    int rc = plan_create(&D->pa, D->nxl, ny, nz, dtype, kPlanExchange);
     if (rc == GPUFFT_SUCCESS) rc = plan_create(&D->pb, nx, D->nyl, nz, dtype, 0);
     if (rc != GPUFFT_SUCCESS) return rc;
     if (exchange) {

@@ -415,9 +415,38 @@ static bool encode_pair_map(CUtensorMap *m, void *data, long long nh, long long 
     return encode_view(m, data, 2 * nh, lines, 2 * nh * 8, box_w, box_h);
 }
 
+// Plans that name no candidate (no autotuning, wisdom or variable) take the
+// one-axis-per-launch kernels over the registered ones where they measured
+// faster (ms per launch or pair of launches, forward + inverse):
+//  * Pass A: the queue form stays at 512^2 planes (512^3 FP32 0.72 against
+//    0.80, FP64 1.50 against 1.56) and at 512 x 128 in FP32, but goes at 512 x
+//    128 in FP64 and at 360 x 240 (R2C + C2R in a row until the 1000 W cap holds
+//    the clock, where the form that crosses HBM less often gains: 1.297 against
+//    1.320, but 2.646 against 2.469, 0.650 against 0.615 and FP64 1.285 against
+//    1.255).  The cluster forms stay for fields
+//    of up to 3 MB, where one launch instead of two is what counts (64^3 0.012
+//    against 0.020; 96^3, 3.6 MB, 0.029 against 0.023; 256^3 0.167 against
+//    0.118; 1024^3 9.68 against 7.51).  (Single launches without the overlap
+//    of axis.cu.)
+//  * x pass: the tensor-copy form stays (512^3 FP32 0.371 against 0.399), as
+//    do short axes and the double-buffered tiles of 128 and 256 points in
+//    FP32 (128 x 512 x 512 0.104 against 0.121); the others go (288^3 0.092
+//    against 0.070, 486^3 0.535 against 0.336, 1024 x 512 x 256 0.447 against
+//    0.396, 128 x 512 x 512 FP64 0.304 against 0.203).
+static bool prefer_axis_a(const Plan &P) {
+    const double bytes = (double)P.nx * P.ny * (P.nz / 2 + 1) * (P.dtype == GPUFFT_FLOAT ? 8 : 16);
+    return P.fa && (P.fa->kind == 2 ? P.fa->m != 256 && !(P.fa->m == 128 && P.dtype == GPUFFT_FLOAT) : bytes > 3e6);
+}
+static bool prefer_axis_b(const Plan &P) {
+    return P.fb && !P.tc_split && P.fb->kind != 3 && P.nx >= 96 &&
+           !(P.dtype == GPUFFT_FLOAT && P.fb->kind == 1 && (P.nx == 128 || P.nx == 256));
+}
+
 // Picks the specialised kernels for this plan's shape (first registry entry,
-// or the entries named by the autotuner) and sizes their launches.
-static int setup_fast(Plan &P, int idx_a, int idx_b) {
+// or the entries named by the autotuner) and sizes their launches.  choose_a,
+// choose_b: the one-axis kernels instead where they are preferred; nothing is
+// then set up, or loaded, of the kernels they replace.
+static int setup_fast(Plan &P, int idx_a, int idx_b, bool choose_a = false, bool choose_b = false) {
     const int vs = P.dtype == GPUFFT_FLOAT ? 8 : 16;
     const fast::VariantA *va = variants_a(P.dtype).data();
     const int na = (int)variants_a(P.dtype).size();
@@ -436,6 +465,17 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
     seen = 0;
     for (int i = 0; i < nb && !P.fb; ++i)
         if (b_eligible(P, vb[i]) && seen++ == idx_b) P.fb = &vb[i];
+    if (P.fa && P.fa->kind == 2 && (!tensor_map_encoder() || P.nx > 32767)) P.fa = nullptr;
+    choose_a = choose_a && prefer_axis_a(P);
+    choose_b = choose_b && prefer_axis_b(P);
+    if (choose_a || choose_b) {
+        const int rc = axis::form_create(P, choose_a, choose_b);
+        if (rc != GPUFFT_SUCCESS) return rc;
+        P.axis_a = choose_a && axis::has_a(P);
+        P.axis_b = choose_b && axis::has_b(P);
+        if (P.axis_a && !(P.exchange && P.fa->kfwd_x)) P.fa = nullptr;
+        if (P.axis_b) P.fb = nullptr;
+    }
     if (P.fa) {
         for (const void *k : {P.fa->kfwd, P.fa->kinv, P.fa->kfwd_x, P.fa->kinv_x}) {
             if (!k) continue;
@@ -447,7 +487,6 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
             }
         }
     }
-    if (P.fa && P.fa->kind == 2 && (!tensor_map_encoder() || P.nx > 32767)) P.fa = nullptr;
     free_queue(P);
     if (P.fa && P.fa->kind == 2) {
         int occ = 0;
@@ -514,45 +553,9 @@ static int setup_fast(Plan &P, int idx_a, int idx_b) {
         const long long tiles = (ncols + P.fb->w - 1) / P.fb->w;
         P.grid_fb = (int)std::min<long long>(tiles, (long long)P.occ_fb * sms);
     }
-    if (!P.fa || (!P.fb && !P.tc_split)) {
-        const int ra = axis::form_create(P);
-        if (ra != GPUFFT_SUCCESS) return ra;
-    }
+    const int ra = axis::form_create(P, !P.fa, !P.fb && !P.tc_split);
+    if (ra != GPUFFT_SUCCESS) return ra;
     return P.dtype == GPUFFT_FLOAT ? upload_stage_tables<float>(P) : upload_stage_tables<double>(P);
-}
-
-// Plans that name no candidate (no autotuning, wisdom or variable) take the
-// one-axis-per-launch kernels over the registered ones where they measured
-// faster (ms per launch or pair of launches, forward + inverse):
-//  * Pass A: the queue form stays at 512^2 planes (512^3 FP32 0.72 against
-//    0.80, FP64 1.50 against 1.56) and at 512 x 128 in FP32, but goes at 512 x
-//    128 in FP64 and at 360 x 240 (R2C + C2R in a row until the 1000 W cap holds
-//    the clock, where the form that crosses HBM less often gains: 1.297 against
-//    1.320, but 2.646 against 2.469, 0.650 against 0.615 and FP64 1.285 against
-//    1.255).  The cluster forms stay for fields
-//    of up to 3 MB, where one launch instead of two is what counts (64^3 0.012
-//    against 0.020; 96^3, 3.6 MB, 0.029 against 0.023; 256^3 0.167 against
-//    0.118; 1024^3 9.68 against 7.51).  (Single launches without the overlap
-//    of axis.cu.)
-//  * x pass: the tensor-copy form stays (512^3 FP32 0.371 against 0.399), as
-//    do short axes and the double-buffered tiles of 128 and 256 points in
-//    FP32 (128 x 512 x 512 0.104 against 0.121); the others go (288^3 0.092
-//    against 0.070, 486^3 0.535 against 0.336, 1024 x 512 x 256 0.447 against
-//    0.396, 128 x 512 x 512 FP64 0.304 against 0.203).
-static int prefer_axis(Plan &P, bool pick_a, bool pick_b) {
-    const double bytes = (double)P.nx * P.ny * (P.nz / 2 + 1) * (P.dtype == GPUFFT_FLOAT ? 8 : 16);
-    bool a = false, b = false;
-    if (pick_a && P.fa)
-        a = P.fa->kind == 2 ? P.fa->m != 256 && !(P.fa->m == 128 && P.dtype == GPUFFT_FLOAT) : bytes > 3e6;
-    if (pick_b && P.fb && !P.tc_split)
-        b = P.fb->kind != 3 && P.nx >= 96 &&
-            !(P.dtype == GPUFFT_FLOAT && P.fb->kind == 1 && (P.nx == 128 || P.nx == 256));
-    if (!a && !b) return GPUFFT_SUCCESS;
-    const int rc = axis::form_create(P);
-    if (rc != GPUFFT_SUCCESS) return rc;
-    P.axis_a = a && axis::has_a(P);
-    P.axis_b = b && axis::has_b(P);
-    return GPUFFT_SUCCESS;
 }
 
 // ---------------------------------------------------------------------------
@@ -867,15 +870,14 @@ static int build_plan(Plan &P) {
     P.occ_b = occ_b;
     if (std::getenv("GPUFFT_GENERIC_ONLY") && !P.tc_split) {
         P.idx_a = P.idx_b = -1;
-        return axis::form_create(P);
+        return axis::form_create(P, true, true);
     }
     int ia = 0, ib = 0;
     if (wisdom_lookup(P, ia, ib, P.kfix)) P.tuned = true;
     const char *va = std::getenv("GPUFFT_VARIANT_A"), *vb = std::getenv("GPUFFT_VARIANT_B");
     if (va) ia = std::atoi(va);
     if (vb) ib = std::atoi(vb);
-    int rc = setup_fast(P, ia, ib);
-    if (rc == GPUFFT_SUCCESS) rc = prefer_axis(P, !P.tuned && !va, !P.tuned && !vb);
+    const int rc = setup_fast(P, ia, ib, !P.tuned && !va, !P.tuned && !vb);
     if (rc == GPUFFT_SUCCESS && P.tc_split && !P.fb)
         return set_error(GPUFFT_ERR_UNSUPPORTED,
                          "no tensor-core x-pass kernel for Nx=%lld (compiled: FP32, Nx = 512 and 1024)", (long long)nx);
@@ -898,6 +900,7 @@ int plan_create(Plan **out, int64_t nx, int64_t ny, int64_t nz, int dtype, int f
     if (!P) return set_error(GPUFFT_ERR_OOM, "host allocation failed");
     P->nx = nx; P->ny = ny; P->nz = nz; P->dtype = dtype;
     P->tc_split = (flags & GPUFFT_PLAN_TC_SPLIT) != 0;
+    P->exchange = (flags & kPlanExchange) != 0;
     if (P->tc_split && dtype != GPUFFT_FLOAT) {
         delete P;
         return set_error(GPUFFT_ERR_UNSUPPORTED, "GPUFFT_PLAN_TC_SPLIT is an FP32 form");
@@ -920,12 +923,8 @@ int plan_adopt(Plan *P, const Plan *Q) {
     if (P->nx != Q->nx || P->ny != Q->ny || P->nz != Q->nz || P->dtype != Q->dtype || P->tc_split != Q->tc_split)
         return set_error(GPUFFT_ERR_INVALID, "plan_adopt: the plans differ in grid or form");
     P->kfix = Q->kfix;
-    int rc = setup_fast(*P, Q->idx_a, Q->idx_b);
-    if (rc == GPUFFT_SUCCESS && (Q->axis_a || Q->axis_b)) rc = axis::form_create(*P);
-    if (rc != GPUFFT_SUCCESS) return rc;
-    P->axis_a = Q->axis_a;
-    P->axis_b = Q->axis_b;
-    P->tuned = Q->tuned;
+    const int rc = setup_fast(*P, Q->idx_a, Q->idx_b, Q->axis_a, Q->axis_b);
+    if (rc == GPUFFT_SUCCESS) P->tuned = Q->tuned;
     return rc;
 }
 
@@ -1199,7 +1198,7 @@ int plan_describe(const Plan *P, char *buf, int len) {
              P->pa.K, P->grid_a, P->occ_a, P->smem_a, P->pa.wz, P->pa.pz, P->pa.wy, P->grid_b, P->occ_b, P->smem_b,
              P->pb.wx, P->pb.ntiles);
     s += b;
-    if (P->fa) {
+    if (P->fa && !P->axis_a) {
         snprintf(b, sizeof(b),
                  " fastA{kind=%d ny=%d m=%d rw=%d wy=%d nt=%d K=%d grid=%d occ=%d smem=%zu depth=%d split=%d}",
                  P->fa->kind, P->fa->ny, P->fa->m, P->fa->rw, P->fa->wy, P->fa->nt, P->k_fa, P->grid_fa, P->occ_fa,

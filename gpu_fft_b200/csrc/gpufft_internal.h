@@ -51,10 +51,11 @@ struct Plan {
     const void *q_unp_i = nullptr;  // inverse pack factors
     const void *q_rtw = nullptr;  // the row FFT's step-1 twiddles
     // one-axis-per-launch kernels (axis.cu), made when a pass has no
-    // specialised kernel or they are the faster choice (axis_a, axis_b: they run
-    // although fa or fb names a kernel; the exchange layout still takes fa's)
+    // specialised kernel or they are the faster choice (axis_a, axis_b).  Then fa
+    // or fb is null, but for the fa of a plan that also runs the exchange layout.
     axis::Form *axis = nullptr;
     bool axis_a = false, axis_b = false;
+    bool exchange = false;
 };
 
 // Programmatic dependent launches (fft_kernels.cuh).  R2C + C2R of a
@@ -84,9 +85,10 @@ inline bool chain_first(const Plan &P, cudaStream_t s) {
 }
 
 namespace axis {
-// Makes P.axis (once): what the passes of this grid need, for those of its
-// lengths that fft_axis.cuh takes (has_a: the z and y axes, has_b: the x axis).
-int form_create(Plan &P);
+// Makes what P's Pass A (a) or x pass (b) needs, once each, if fft_axis.cuh
+// takes its lengths (has_a: the z and y axes, has_b: the x axis).  Only the
+// passes that will run: their kernels are loaded here.
+int form_create(Plan &P, bool a, bool b);
 void form_destroy(Plan &P);
 bool has_a(const Plan &P);
 bool has_b(const Plan &P);
@@ -108,6 +110,8 @@ bool encode_view(CUtensorMap *m, void *data, long long width, long long lines, l
 struct DistPlan;
 int dist_exec(DistPlan *D, void *data, cudaStream_t s, bool fwd);
 void dist_free(DistPlan *D);
+// (kPlanExchange among the flags: the plan also runs its Pass A in the exchange layout)
+constexpr int kPlanExchange = 1 << 30;
 int plan_create(Plan **out, int64_t nx, int64_t ny, int64_t nz, int dtype, int flags);
 int plan_destroy(Plan *P);
 int plan_exec(const Plan *P, void *data, void *stream, bool forward);

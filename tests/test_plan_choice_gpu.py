@@ -40,3 +40,17 @@ def test_a_plan_adopts_the_choice_of_no_registered_kernel(cuda, tmp_path):
     p.r2c(a)
     q.r2c(b)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("grid, runs, tables", [((108, 512, 256), {"fastA", "axisX"}, 108 * 8),
+                                                ((384, 512, 512), {"fastA", "fastB"}, 0),
+                                                ((48, 360, 480), {"axisZ", "axisY", "fastB"}, (360 + 240 + 2 * 121) * 8),
+                                                ((54, 54, 54), {"fastA", "fastB"}, 0)], ids=str)
+def test_a_plan_makes_and_names_only_what_it_runs(cuda, grid, runs, tables):
+    """Default plans in FP32: no tables for an axis that a registered kernel
+    takes, and no registered kernel beside the one-axis kernels that replace it."""
+    import gpu_fft_b200 as g
+
+    d = g.Plan(*grid, "float").describe()
+    assert {k for k in ("fastA", "fastB", "axisX", "axisY", "axisZ") if k + "{" in d} == runs, d
+    assert (f" axisTables={tables}" in d) if tables else ("axisTables" not in d), d
