@@ -20,7 +20,7 @@ SOURCES = ["gpufft.cu", "fast_f32.cu", "fast_f64.cu", "noalloc.cu", "batch.cu", 
            "axis.cu"]
 # sources compiled several times: (source, object name, definitions)
 PARTS = [("axis_kernels.cu", f"axis_kernels_{d}_{i}.o", [f"-DGPUFFT_AXIS_F64={d}", f"-DGPUFFT_AXIS_PART={i}"])
-         for d in (1, 0) for i in range(16)]
+         for d in (1, 0) for i in range(64)]
 HEADERS = ["fft_axis.cuh", "axis_lengths.h", "fft_kernels.cuh", "fft_radix.cuh", "fft_fast.cuh", "fft_s16.cuh", "fft_queue.cuh", "fast_registry.h", "fast_entries.h", "gpufft_internal.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2", "-Xfatbin=-compress-all"]
