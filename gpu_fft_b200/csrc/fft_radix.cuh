@@ -539,6 +539,25 @@ template <int A, int B, bool FWD, typename V> struct DftPfa {
         }
     }
 };
+// x * exp(s*2*pi*i*m/R) for an m known when the loops are unrolled.  Rounded to
+// FP32, the constants of R = 32 all have moduli below 1 (by up to 2.9e-8), so
+// that their errors add up over the stages: the larger one of each is carried
+// on by one more FMA a component.  1024 points (32 x 32) in FP32, emulated:
+// 1.117e-7 -> 1.036e-7 from the exact result, 16 x 8 x 8 1.081e-7.
+template <int R, bool FWD, typename V> __device__ __forceinline__ V tw_const(V a, int m) {
+    using T = decltype(a.x);
+    const double cd = Trig<R>::c(m), td = FWD ? -Trig<R>::s(m) : Trig<R>::s(m);
+    const T c = (T)cd, t = (T)td;
+    if constexpr (R == 32 && sizeof(T) == 4) {
+        if (cd * cd >= td * td) {
+            const T l = (T)(cd - (double)c);
+            return V{fmaf(a.x, c, fmaf(a.x, l, -(a.y * t))), fmaf(a.y, c, fmaf(a.y, l, a.x * t))};
+        }
+        const T l = (T)(td - (double)t);
+        return V{fmaf(-a.y, t, fmaf(-a.y, l, a.x * c)), fmaf(a.x, t, fmaf(a.x, l, a.y * c))};
+    }
+    return V{a.x * c - a.y * t, a.x * t + a.y * c};
+}
 // R = A B: DFT_A over n1 of x[B n1 + n2] for each n2, twiddle w_R^(n2 k1),
 // DFT_B over n2 for each k1, output k = k1 + A k2
 template <int A, int B, bool FWD, typename V> struct DftCt {
@@ -560,8 +579,7 @@ template <int A, int B, bool FWD, typename V> struct DftCt {
                 } else if (4 * m == R) {
                     y[k1][n2] = c_rot<FWD>(a[k1]);
                 } else {
-                    const T c = (T)Trig<R>::c(m), t = FWD ? -(T)Trig<R>::s(m) : (T)Trig<R>::s(m);
-                    y[k1][n2] = V{a[k1].x * c - a[k1].y * t, a[k1].x * t + a[k1].y * c};
+                    y[k1][n2] = tw_const<R, FWD>(a[k1], m);
                 }
             }
         }
