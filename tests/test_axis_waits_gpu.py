@@ -78,3 +78,51 @@ def test_axis_wait_runs_out_and_reports(cuda, which, dt, monkeypatch):
     _noalloc(g, grid, dt, True, want)
     assert _rel(a, want) < _tol(grid, dt)
     q.check()
+
+
+@pytest.mark.parametrize("before", ["kernel", "copy", "other stream", "transform"])
+@pytest.mark.parametrize("n, dt", [(32, "float"), (64, "float"), (100, "float"), (128, "float"), (100, "double")])
+def test_launches_of_a_transform_keep_their_order(cuda, n, dt, before):
+    """A transform's first launch may start while what is before it in the
+    stream drains, and its kernels let the next one in early: the field written
+    immediately before (by a kernel, a copy, another stream's kernel, or the
+    inverse transform of another plan) and read immediately after, many times
+    without a pause on a stream of its own, gives the bits of calls waited for."""
+    import torch
+    import gpu_fft_b200 as g
+
+    grid = (n, n, n)
+    p, q = g.Plan(*grid, dt), g.Plan(*grid, dt)
+    src = [_make(grid, dt, s) for s in (1, 2)]
+    f, out, want = torch.empty_like(src[0]), torch.empty_like(src[0]), []
+    for x in src:
+        f.copy_(x)
+        torch.cuda.synchronize()
+        if before == "transform":
+            q.c2r(f)
+            torch.cuda.synchronize()
+        p.r2c(f)
+        torch.cuda.synchronize()
+        want.append(f.clone())
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    here, there = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(here):
+        for k in range(200):
+            x = src[k % 2]
+            if before == "other stream":
+                there.wait_stream(here)
+                with torch.cuda.stream(there):
+                    torch.mul(x, 1.0, out=f)
+                here.wait_stream(there)
+            elif before == "copy":
+                f.copy_(x)
+            else:
+                torch.mul(x, 1.0, out=f)
+            if before == "transform":
+                q.c2r(f)
+            p.r2c(f)
+            torch.mul(f, 1.0, out=out)
+            wrong += (out != want[k % 2]).any()
+    torch.cuda.synchronize()
+    assert wrong.item() == 0
