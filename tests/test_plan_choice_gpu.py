@@ -3,7 +3,7 @@ import ctypes
 
 import pytest
 
-from test_axis_gpu import _make
+from test_axis_gpu import _make, _noalloc, _rel, _tol
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +54,27 @@ def test_a_plan_makes_and_names_only_what_it_runs(cuda, grid, runs, tables):
     d = g.Plan(*grid, "float").describe()
     assert {k for k in ("fastA", "fastB", "axisX", "axisY", "axisZ") if k + "{" in d} == runs, d
     assert (f" axisTables={tables}" in d) if tables else ("axisTables" not in d), d
+
+
+@pytest.mark.parametrize("grid, dt", [((64, 64, 64), "float"), ((128, 128, 128), "float"), ((512, 512, 512), "float"),
+                                      ((256, 128, 64), "float"), ((128, 128, 128), "double")], ids=str)
+def test_registered_kernels_agree_with_the_runtime_radix_kernels(cuda, grid, dt, monkeypatch):
+    """The registered kernels of both passes, named (a default plan may take
+    the one-axis kernels), against gpufft_exec_noalloc, which runs the
+    runtime-radix kernels."""
+    import torch
+    import gpu_fft_b200 as g
+
+    monkeypatch.setenv("GPUFFT_VARIANT_A", "0")
+    monkeypatch.setenv("GPUFFT_VARIANT_B", "0")
+    p = g.Plan(*grid, dt)
+    d = p.describe()
+    assert "fastA{" in d and "fastB{" in d and "axis" not in d
+    a = _make(grid, dt, 3)
+    for forward in (True, False):
+        b = a.clone()
+        (p.r2c if forward else p.c2r)(a)
+        _noalloc(g, grid, dt, forward, b)
+        x, y = (a, b) if forward else (a[..., :grid[2]], b[..., :grid[2]])
+        assert _rel(x, y) < _tol(grid, dt)
+        a = b
