@@ -1,6 +1,7 @@
 // axis.cu — plans and launches of the one-axis-per-launch kernels
-// (fft_axis.cuh): the general path, taken by every pass that has no entry in
-// the registry of specialised kernels (gpufft.cu) and whose lengths they take.
+// (fft_axis.cuh): taken by every pass whose lengths they take and that has no
+// entry in the registry of specialised kernels or is faster on these (the rule
+// of prefer_axis_a and prefer_axis_b in gpufft.cu).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>

@@ -15,9 +15,10 @@
 //    radices, and registers that fit the radices;
 //  * a thread keeps its butterflies in registers, so a stage works in place;
 //  * a tile is W sequences, element (i, w) at i * PW + w: a half-warp reads
-//    and writes W adjacent elements (128 bytes) whatever the radix, so no
-//    stage has bank conflicts.  Rows (z) use PW = W + 1, which makes their
-//    turning over conflict-free too;
+//    and writes W adjacent elements (128 bytes) whatever the radix, without
+//    bank conflicts.  Rows (z) use PW = W + 1, so that turning them over has
+//    none either (ncu counts 10-13% of all shared wavefronts as conflicts in
+//    the column kernels, 12-16% in the rows');
 //  * tiles are copied in ahead of use by tensor copies (columns) and one bulk
 //    copy (rows): against cp.async 20% fewer instructions and 40% fewer
 //    shared-memory wavefronts (500^3 FP32 x axis 215 -> 177 us, z and y axes
@@ -25,9 +26,10 @@
 // z and y run as two launches, so the field crosses HBM three times per
 // transform instead of twice (from L2 when it fits there); what that costs is
 // less than what the instructions saved bring: R2C + C2R of 420 x 378 x 500
-// FP32 2.01 -> 0.77 ms, 768^3 12.4 -> 4.4, 225 x 243 x 350 FP64 0.86 -> 0.42.
-// Each launch moves 0.7-0.85 of the copy bandwidth; issue slots are 35-40%
-// used and no pipe is over 45%: what is left is waiting at the block barriers
+// FP32 2.01 -> 0.75 ms, 768^3 12.4 -> 4.2, 225 x 243 x 350 FP64 0.86 -> 0.35.
+// Each launch moves 0.7-0.85 of the copy bandwidth; at 252 x 378 x 500 FP32
+// 34-43% of the issue slots are used, the FMA pipe 27-37%, the shared-memory
+// data pipe 36-37% (rows 60%): what is left is waiting at the block barriers
 // between a stage's bursts of shared-memory accesses and its arithmetic.
 #pragma once
 #include "fft_fast.cuh"

@@ -190,7 +190,7 @@ __device__ __forceinline__ void stage(const cx_t<T> *__restrict__ src, cx_t<T> *
 #pragma unroll
             for (int j = 1; j < R; ++j) v[j] = c_tw<FWD>(v[j], tw[j * e]);
         }
-        Dft<R, FWD, V>::run(v);
+        DftRuntime<R, FWD, V>::run(v);
         V *out = dst + (ip * p * R + k) * sn + w * sw;
 #pragma unroll
         for (int j = 0; j < R; ++j) out[j * ostride] = v[j];

@@ -417,22 +417,27 @@ static bool encode_pair_map(CUtensorMap *m, void *data, long long nh, long long 
 
 // Plans that name no candidate (no autotuning, wisdom or variable) take the
 // one-axis-per-launch kernels over the registered ones where they measured
-// faster (ms per launch or pair of launches, forward + inverse):
-//  * Pass A: the queue form stays at 512^2 planes (512^3 FP32 0.72 against
-//    0.80, FP64 1.50 against 1.56) and at 512 x 128 in FP32, but goes at 512 x
-//    128 in FP64 and at 360 x 240 (R2C + C2R in a row until the 1000 W cap holds
-//    the clock, where the form that crosses HBM less often gains: 1.297 against
-//    1.320, but 2.646 against 2.469, 0.650 against 0.615 and FP64 1.285 against
-//    1.255).  The cluster forms stay for fields
-//    of up to 3 MB, where one launch instead of two is what counts (64^3 0.012
-//    against 0.020; 96^3, 3.6 MB, 0.029 against 0.023; 256^3 0.167 against
-//    0.118; 1024^3 9.68 against 7.51).  (Single launches without the overlap
-//    of axis.cu.)
-//  * x pass: the tensor-copy form stays (512^3 FP32 0.371 against 0.399), as
-//    do short axes and the double-buffered tiles of 128 and 256 points in
-//    FP32 (128 x 512 x 512 0.104 against 0.121); the others go (288^3 0.092
-//    against 0.070, 486^3 0.535 against 0.336, 1024 x 512 x 256 0.447 against
-//    0.396, 128 x 512 x 512 FP64 0.304 against 0.203).
+// faster.  R2C + C2R in a row with the overlap of launches that both have, us,
+// registered against one-axis:
+//  * Pass A: the queue form stays at 512^2 planes (512^3 FP32 1090 against 1204,
+//    FP64 2290 against 2316) and at 512 x 128 in FP32, but goes at 512 x 128 in
+//    FP64 (2645 against 2328) and at 360 x 240 (638 against 590, FP64 1245
+//    against 1223).  At 512 x 128 in FP32 a burst is faster on the one-axis
+//    kernels (1283 against 1239), but after some seconds in a row, when the 1000 W
+//    cap holds the clock, the queue form, which crosses HBM less often (1304
+//    against 1343; 512 x 512 x 256 661 against 680).  The cluster forms stay for fields of up to 3 MB, where one launch instead of two
+//    counts (64^3, 1.1 MB, 12.0 against 17.0; 24 x 128 x 128 16.6 against 23.3; 64 x
+//    128 x 64, 2.2 MB, 14.7 against 21.7).  About the line it depends on the plane:
+//    72^3, 1.5 MB, 20.5 against 18.8; 48 x 128 x 128, 3.2 MB, 26.0 against 27.1; 96^3,
+//    3.6 MB, 33.3 against 26.5; from there on the one-axis kernels (144^3 72 against
+//    37, 256^3 206 against 150).
+//  * x pass: the tensor-copy form stays (512^3 FP32 1089 against 1124), as do axes
+//    below 96 points (72 x 64 x 64 17.4 against 18.4, but 72 x 512 x 512 203
+//    against 164) and the double-buffered tiles of 128 and 256 points in FP32
+//    (128 x 512 x 512 294 against 310, 256 x 512 x 512 574 against 569); the others
+//    go (144 x 256 x 256 106 against 92, 96 x 256 x 256 80 against 71, though 96 x
+//    64 x 64 19.0 against 20.1; FP64 128 x 256 x 256 139 against 124, 1024 x 256 x
+//    256 1267 against 1232).
 static bool prefer_axis_a(const Plan &P) {
     const double bytes = (double)P.nx * P.ny * (P.nz / 2 + 1) * (P.dtype == GPUFFT_FLOAT ? 8 : 16);
     return P.fa && (P.fa->kind == 2 ? P.fa->m != 256 && !(P.fa->m == 128 && P.dtype == GPUFFT_FLOAT) : bytes > 3e6);
