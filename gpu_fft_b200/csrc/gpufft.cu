@@ -433,17 +433,21 @@ static bool encode_pair_map(CUtensorMap *m, void *data, long long nh, long long 
 //    37, 256^3 206 against 150).
 //  * x pass: the tensor-copy form stays (512^3 FP32 1089 against 1124), as do axes
 //    below 96 points (72 x 64 x 64 17.4 against 18.4, but 72 x 512 x 512 203
-//    against 164) and the double-buffered tiles of 128 and 256 points in FP32
-//    (128 x 512 x 512 294 against 310, 256 x 512 x 512 574 against 569); the others
-//    go (144 x 256 x 256 106 against 92, 96 x 256 x 256 80 against 71, though 96 x
-//    64 x 64 19.0 against 20.1; FP64 128 x 256 x 256 139 against 124, 1024 x 256 x
-//    256 1267 against 1232).
+//    against 164), the double-buffered tiles of 128 and 256 points in FP32 (128 x
+//    512 x 512 294 against 310, 256 x 512 x 512 574 against 569) and fields of up to
+//    9 MB (96^3, 3.6 MB, 24.5 against 26.3; 108 x 64 x 64 19.0 against 21.5; FP64
+//    1024 x 32 x 32, 8.9 MB, 38.4 against 39.4; but 108 x 128 x 128, 7.2 MB, 35.2
+//    against 34.1); the others go (144 x 128 x 128, 9.6 MB, 40.1 against 39.1; 144 x
+//    256 x 256 106 against 92; 96 x 256 x 256 80 against 71; FP64 128 x 256 x 256 139
+//    against 124, 1024 x 256 x 256 1267 against 1232).
+static double field_bytes_of(const Plan &P) {
+    return (double)P.nx * P.ny * (P.nz / 2 + 1) * (P.dtype == GPUFFT_FLOAT ? 8 : 16);
+}
 static bool prefer_axis_a(const Plan &P) {
-    const double bytes = (double)P.nx * P.ny * (P.nz / 2 + 1) * (P.dtype == GPUFFT_FLOAT ? 8 : 16);
-    return P.fa && (P.fa->kind == 2 ? P.fa->m != 256 && !(P.fa->m == 128 && P.dtype == GPUFFT_FLOAT) : bytes > 3e6);
+    return P.fa && (P.fa->kind == 2 ? P.fa->m != 256 && !(P.fa->m == 128 && P.dtype == GPUFFT_FLOAT) : field_bytes_of(P) > 3e6);
 }
 static bool prefer_axis_b(const Plan &P) {
-    return P.fb && !P.tc_split && P.fb->kind != 3 && P.nx >= 96 &&
+    return P.fb && !P.tc_split && P.fb->kind != 3 && P.nx >= 96 && field_bytes_of(P) > 9e6 &&
            !(P.dtype == GPUFFT_FLOAT && P.fb->kind == 1 && (P.nx == 128 || P.nx == 256));
 }
 

@@ -45,7 +45,10 @@ def test_a_plan_adopts_the_choice_of_no_registered_kernel(cuda, tmp_path):
 @pytest.mark.parametrize("grid, runs, tables", [((108, 512, 256), {"fastA", "axisX"}, 108 * 8),
                                                 ((384, 512, 512), {"fastA", "fastB"}, 0),
                                                 ((48, 360, 480), {"axisZ", "axisY", "fastB"}, (360 + 240 + 2 * 121) * 8),
-                                                ((54, 54, 54), {"fastA", "fastB"}, 0)], ids=str)
+                                                ((54, 54, 54), {"fastA", "fastB"}, 0),
+                                                ((96, 96, 96), {"axisZ", "axisY", "fastB"}, (96 + 48 + 2 * 25) * 8),
+                                                ((96, 192, 160), {"axisX", "axisY", "axisZ"}, (96 + 192 + 80 + 2 * 41) * 8)],
+                         ids=str)
 def test_a_plan_makes_and_names_only_what_it_runs(cuda, grid, runs, tables):
     """Default plans in FP32: no tables for an axis that a registered kernel
     takes, and no registered kernel beside the one-axis kernels that replace it."""
