@@ -378,14 +378,14 @@ template <bool FWD, typename V> struct Dft<8, FWD, V> {
         // even/odd split: E = DFT4(x0,x2,x4,x6), O = DFT4(x1,x3,x5,x7); y[k] = E[k] + w8^k O[k]
         dft4<FWD>(x[0], x[2], x[4], x[6]);
         dft4<FWD>(x[1], x[3], x[5], x[7]);
-        V o1 = tw16<FWD, 2>(x[3]), o2 = x[5], o3 = tw16<FWD, 6>(x[7]);
+        V o1 = tw16<FWD, 2>(x[3]), o2 = tw16<FWD, 4>(x[5]), o3 = tw16<FWD, 6>(x[7]);
         V e0 = x[0], e1 = x[2], e2 = x[4], e3 = x[6], o0 = x[1];
         x[0] = c_add(e0, o0);
         x[4] = c_sub(e0, o0);
         x[1] = c_add(e1, o1);
         x[5] = c_sub(e1, o1);
-        x[2] = c_addi<!FWD>(e2, o2);
-        x[6] = c_addi<FWD>(e2, o2);
+        x[2] = c_add(e2, o2);
+        x[6] = c_sub(e2, o2);
         x[3] = c_add(e3, o3);
         x[7] = c_sub(e3, o3);
     }
