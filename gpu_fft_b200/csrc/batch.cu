@@ -91,13 +91,13 @@ __device__ void batch_plane(const BatchDesc &D, int x, unsigned char *smem) {
     V *g = reinterpret_cast<V *>(P.data) + (long long)x * P.ny * P.nh;
     const int ntiles_y = (P.m + P.wy - 1) / P.wy;
     if (D.forward) {
-        for (int r0 = 0; r0 < P.ny; r0 += P.wz) rows_r2c<T>(P, g, ta, tb, twz, r0, min(P.wz, P.ny - r0));
+        for (int r0 = 0; r0 < P.ny; r0 += P.wz) rows_r2c<T, true>(P, g, ta, tb, twz, r0, min(P.wz, P.ny - r0));
         __syncthreads();
-        for (int t = 0; t < ntiles_y; ++t) cols_y<T, true>(P, g, ta, tb, twy, t * P.wy, min(P.wy, P.m - t * P.wy));
+        for (int t = 0; t < ntiles_y; ++t) cols_y<T, true, true>(P, g, ta, tb, twy, t * P.wy, min(P.wy, P.m - t * P.wy));
     } else {
-        for (int t = 0; t < ntiles_y; ++t) cols_y<T, false>(P, g, ta, tb, twy, t * P.wy, min(P.wy, P.m - t * P.wy));
+        for (int t = 0; t < ntiles_y; ++t) cols_y<T, false, true>(P, g, ta, tb, twy, t * P.wy, min(P.wy, P.m - t * P.wy));
         __syncthreads();
-        for (int r0 = 0; r0 < P.ny; r0 += P.wz) rows_c2r<T>(P, g, ta, tb, twz, r0, min(P.wz, P.ny - r0));
+        for (int r0 = 0; r0 < P.ny; r0 += P.wz) rows_c2r<T, true>(P, g, ta, tb, twz, r0, min(P.wz, P.ny - r0));
     }
 }
 
@@ -115,8 +115,8 @@ __device__ void batch_tile(const BatchDesc &D, long long tile, unsigned char *sm
     const int wv = (int)min((long long)P.wx, P.ncols - c0);
     load_cols<T>(ta, base + c0, P.ncols, P.nx, P.wx, P.wxdiv, wv);
     __syncthreads();
-    V *res = D.forward ? fft_tile<T, true>(ta, tb, P.wx, 1, P.wx, P.wxdiv, P.ax, twx)
-                       : fft_tile<T, false>(ta, tb, P.wx, 1, P.wx, P.wxdiv, P.ax, twx);
+    V *res = D.forward ? fft_tile<T, true, true>(ta, tb, P.wx, 1, P.wx, P.wxdiv, P.ax, twx)
+                       : fft_tile<T, false, true>(ta, tb, P.wx, 1, P.wx, P.wxdiv, P.ax, twx);
     store_cols<T>(res, base + c0, P.ncols, P.nx, P.wx, P.wxdiv, 0, wv);
 }
 

@@ -168,7 +168,7 @@ template <> struct MaxE<double> { static constexpr int value = 16; };
 // tile at s[n*sn + w*sw].  Each thread walks its butterflies one at a time,
 // so only R complex values are live per thread whatever the radix.
 // ---------------------------------------------------------------------------
-template <typename T, int R, bool FWD>
+template <typename T, int R, bool FWD, bool PACKED>
 __device__ __forceinline__ void stage(const cx_t<T> *__restrict__ src, cx_t<T> *__restrict__ dst, int sn, int sw,
                                       int W, const FastDiv &wdiv, int n, int p, const FastDiv &pdiv, int twstep,
                                       const cx_t<T> *tw) {
@@ -190,7 +190,7 @@ __device__ __forceinline__ void stage(const cx_t<T> *__restrict__ src, cx_t<T> *
 #pragma unroll
             for (int j = 1; j < R; ++j) v[j] = c_tw<FWD>(v[j], tw[j * e]);
         }
-        DftRuntime<R, FWD, V>::run(v);
+        DftRuntime<R, FWD, V, PACKED>::run(v);
         V *out = dst + (ip * p * R + k) * sn + w * sw;
 #pragma unroll
         for (int j = 0; j < R; ++j) out[j * ostride] = v[j];
@@ -199,23 +199,23 @@ __device__ __forceinline__ void stage(const cx_t<T> *__restrict__ src, cx_t<T> *
 
 // Runs all stages of `ax`, ping-ponging between a and b; returns the tile
 // that holds the result.  Ends with a block barrier.
-template <typename T, bool FWD>
+template <typename T, bool FWD, bool PACKED>
 __device__ __forceinline__ cx_t<T> *fft_tile(cx_t<T> *a, cx_t<T> *b, int sn, int sw, int W, const FastDiv &wdiv,
                                              const AxisPlan &ax, const cx_t<T> *tw) {
     for (int st = 0; st < ax.nst; ++st) {
         const int p = ax.p[st], tws = ax.twstep[st];
         const FastDiv pd = ax.pdiv[st];
         switch (ax.radix[st]) {
-            case 2: stage<T, 2, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 3: stage<T, 3, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 4: stage<T, 4, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 5: stage<T, 5, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 7: stage<T, 7, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 8: stage<T, 8, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 9: stage<T, 9, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 11: stage<T, 11, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 13: stage<T, 13, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
-            case 16: stage<T, 16, FWD>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 2: stage<T, 2, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 3: stage<T, 3, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 4: stage<T, 4, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 5: stage<T, 5, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 7: stage<T, 7, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 8: stage<T, 8, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 9: stage<T, 9, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 11: stage<T, 11, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 13: stage<T, 13, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
+            case 16: stage<T, 16, FWD, PACKED>(a, b, sn, sw, W, wdiv, ax.n, p, pd, tws, tw); break;
             default: break;  // the plan only emits the radices above
         }
         __syncthreads();
@@ -279,7 +279,7 @@ __device__ __forceinline__ void store_rows(const PassAParams &P, cx_t<T> *dst, c
 }
 
 // Forward rows [r0, r0+wv) of plane g: z-axis R2C.
-template <typename T>
+template <typename T, bool PACKED = false>
 __device__ void rows_r2c(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> *tb, const cx_t<T> *twz, int r0,
                          int wv) {
     using V = cx_t<T>;
@@ -287,7 +287,7 @@ __device__ void rows_r2c(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> 
     load_rows<T>(P, g + (long long)r0 * P.nh, ta, wv);
     __syncthreads();
     // m-point complex FFT of every row: z[n] = x[2n] + i x[2n+1]
-    V *res = fft_tile<T, true>(ta, tb, 1, pz, W, P.wzdiv, P.az, twz);
+    V *res = fft_tile<T, true, PACKED>(ta, tb, 1, pz, W, P.wzdiv, P.az, twz);
     V *out = (res == ta) ? tb : ta;
     // unpack: X[k] = E + O, X[m-k] = conj(E - O),  E = (Z[k] + conj Z[m-k])/2,
     // O = -i w^k (Z[k] - conj Z[m-k])/2,  w = exp(-2 pi i / Nz); k = 0..m/2.
@@ -317,7 +317,7 @@ __device__ void rows_r2c(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> 
 }
 
 // Inverse rows: z-axis C2R.  Slot 0 holds (Re X0, Re X_m) packed by cols_y<inverse>.
-template <typename T>
+template <typename T, bool PACKED = false>
 __device__ void rows_c2r(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> *tb, const cx_t<T> *twz, int r0,
                          int wv) {
     using V = cx_t<T>;
@@ -346,7 +346,7 @@ __device__ void rows_c2r(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> 
         if (k != 0 && m - k != k) tb[w * pz + m - k] = c_conj(c_sub(s, pk));
     }
     __syncthreads();
-    V *res = fft_tile<T, false>(tb, ta, 1, pz, W, P.wzdiv, P.az, twz);
+    V *res = fft_tile<T, false, PACKED>(tb, ta, 1, pz, W, P.wzdiv, P.az, twz);
     // slot m is padding of the real row (cells Nz, Nz+1): written as zero
     for (int q = threadIdx.x; q < W; q += kThreads) res[q * pz + m] = V{(T)0, (T)0};
     __syncthreads();
@@ -355,7 +355,7 @@ __device__ void rows_c2r(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> 
 }
 
 // y-axis FFT of columns [c0, c0+wv) of plane g (columns 0..m-1; column 0 packed).
-template <typename T, bool FWD>
+template <typename T, bool FWD, bool PACKED = false>
 __device__ void cols_y(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> *tb, const cx_t<T> *twy, int c0,
                        int wv) {
     using V = cx_t<T>;
@@ -379,7 +379,7 @@ __device__ void cols_y(const PassAParams &P, cx_t<T> *g, cx_t<T> *ta, cx_t<T> *t
         }
         __syncthreads();
     }
-    V *res = fft_tile<T, FWD>(ta, tb, W, 1, W, P.wydiv, P.ay, twy);
+    V *res = fft_tile<T, FWD, PACKED>(ta, tb, W, 1, W, P.wydiv, P.ay, twy);
     if (FWD && c0 == 0) {
         // column 0 carried a (bin 0) + i b (bin m), both real along y:
         // A[ky] = (C[ky] + conj C[-ky]) / 2,  B[ky] = -i (C[ky] - conj C[-ky]) / 2
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(kThreads) pass_b_kernel(PassBParams P) {
         const int wv = (int)min((long long)P.wx, P.ncols - c0);
         load_cols<T>(ta, base + c0, P.ncols, P.nx, P.wx, P.wxdiv, wv);
         __syncthreads();
-        V *res = fft_tile<T, FWD>(ta, tb, P.wx, 1, P.wx, P.wxdiv, P.ax, twx);
+        V *res = fft_tile<T, FWD, false>(ta, tb, P.wx, 1, P.wx, P.wxdiv, P.ax, twx);
         if (P.epi) {
             for (int q = threadIdx.x; q < P.nx * P.wx; q += kThreads) {
                 const int r = (int)fdiv((uint32_t)q, P.wxdiv);

@@ -517,11 +517,14 @@ template <bool FWD, typename V> struct Dft<11, FWD, V> : DftOdd<11, FWD, V> {};
 template <bool FWD, typename V> struct Dft<13, FWD, V> : DftOdd<13, FWD, V> {};
 
 // The DFTs of a kernel that switches over the radices at run time: all of them
-// share one kernel's registers, and packed FMAs in the odd ones took the FP32 x
-// pass from 52 to 59 (2 x 400 x 500 12.8 against 14.4 us a launch, 12 x 1000 x 1000
-// 88 against 94).
-template <int R, bool FWD, typename V>
-using DftRuntime = std::conditional_t<R == 3 || R == 5 || R == 7 || R == 11 || R == 13, DftOdd<R, FWD, V, false>, Dft<R, FWD, V>>;
+// share one kernel's registers.  In the kernels of one pass packed FMAs in the
+// odd radices lose (FP32 x pass 59 registers against 52: 2 x 400 x 500 14.4 us a
+// launch against 12.8, 12 x 1000 x 1000 94 against 88), in the batch kernel, which
+// runs both passes and directions, they gain (24 R2C of 64^3 86 us against 106, 8
+// of 100^3 118 against 145, of 243 x 243 x 250 503 against 549).
+template <int R, bool FWD, typename V, bool PACKED>
+using DftRuntime = std::conditional_t<!PACKED && (R == 3 || R == 5 || R == 7 || R == 11 || R == 13),
+                                      DftOdd<R, FWD, V, false>, Dft<R, FWD, V>>;
 
 // R = A B with gcd(A, B) = 1 by the prime-factor (Good-Thomas) map, no
 // twiddles: input n = (B n1 + A n2) mod R, output k = (B (1/B mod A) k1 +

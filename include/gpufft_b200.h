@@ -95,8 +95,13 @@ int gpufft_plan_destroy(gpufft_plan plan);
  * a bounded wait inside one of its kernels ran out since the plan was made
  * (the queue-scheduled Pass A waiting for a plane, the tensor-core x pass
  * waiting for its MMAs, or a one-axis kernel waiting for a tile's copy; the
- * results of that call are wrong and the plan should be destroyed), else GPUFFT_SUCCESS.  No reference counterpart. */
+ * results of that call are wrong and the plan should be destroyed), else
+ * GPUFFT_SUCCESS.  No reference counterpart. */
 int gpufft_plan_check(gpufft_plan plan);
+/* In place, ordered with the work before and after on `stream`; may be
+ * captured into a graph.  The edges between one transform's kernel nodes are
+ * then programmatic ones, for which cudaGraphGetEdges without edge data
+ * answers cudaErrorLossyQuery (use the form with edge data). */
 int gpufft_exec_r2c(gpufft_plan plan, void *data, void *stream);
 int gpufft_exec_c2r(gpufft_plan plan, void *data, void *stream);
 /* The same with an epilogue fused into the x pass, for pseudo-spectral steps
