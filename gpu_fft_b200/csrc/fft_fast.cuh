@@ -615,7 +615,7 @@ __device__ __forceinline__ void pass_b_fast_run(const PassBParams &P, unsigned c
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = base + c0;
         static_assert(NT % W == 0, "a thread's elements are of one column");
-        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
+        const PassBEpilogue<T, FWD> epi(P, c0 + threadIdx.x % W);
         auto src = [&](int n, int w) -> V {
             return (w < wv) ? ld_g(g + (long long)n * ncols + w) : V{(T)0, (T)0};
         };
@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(NT, MINB) pass_b_pipe(PassBParams P) {
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = obase + c0;
         static_assert(NT % W == 0, "a thread's elements are of one column");
-        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
+        const PassBEpilogue<T, FWD> epi(P, c0 + threadIdx.x % W);
         auto dst = [&](int n, int w, V v) {
             if (w < wv) {
                 if constexpr (EPI)
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(NT, MINB) pass_b_pipe1(PassBParams P) {
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = obase + c0;
         static_assert(NT % W == 0, "a thread's elements are of one column");
-        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
+        const PassBEpilogue<T, FWD> epi(P, c0 + threadIdx.x % W);
         auto dst = [&](int n, int w, V v) {
             if (w < wv) {
                 if constexpr (EPI)

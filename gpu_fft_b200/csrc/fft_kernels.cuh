@@ -122,21 +122,23 @@ __device__ __forceinline__ V pass_b_epilogue(const PassBParams &P, V v, int kx, 
 // The same for kernels whose threads keep one column of a tile: what depends
 // on the column is worked out once per tile.  (Per element, the double-to-float
 // conversion of the scale and the division by Nh took the 512^3 FP32 x pass
-// from 185 to 288 us with a scale and 425 with the mask.)
-template <typename T>
+// from 185 to 288 us with a scale and 425 with the mask.)  The inverse (FWD
+// false) has no mask, and none of its tests (scaled C2R in FP64, 384 x 360 x 480
+// 608 us against 611, 512^3 1180 against 1182).
+template <typename T, bool FWD>
 struct PassBEpilogue {
     T scale;
     int nx;     // 0 without the mask
     bool drop;  // ky or kz outside the box
     __device__ __forceinline__ PassBEpilogue(const PassBParams &P, long long col)
-        : scale((T)P.scale), nx(P.dealias ? P.nx : 0), drop(false) {
-        if (nx) {
+        : scale((T)P.scale), nx(FWD && P.dealias ? P.nx : 0), drop(false) {
+        if (FWD && nx) {
             const int c = (int)col, ky = c / P.nh, kz = c - ky * P.nh;
             drop = 3 * min(ky, P.ny - ky) > P.ny || 3 * kz > P.nz;
         }
     }
     template <typename V> __device__ __forceinline__ V operator()(V v, int kx) const {
-        if (nx && (drop || 3 * min(kx, nx - kx) > nx)) return V{(T)0, (T)0};
+        if (FWD && nx && (drop || 3 * min(kx, nx - kx) > nx)) return V{(T)0, (T)0};
         return V{v.x * scale, v.y * scale};
     }
 };

@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(NT, 1) pass_b_tma(const PassBParams P, const _
         const int wv = (int)min((long long)W, ncols - c0);
         V *g = base + c0;
         static_assert(NT % W == 0, "a thread's elements are of one column");
-        const PassBEpilogue<T> epi(P, c0 + threadIdx.x % W);
+        const PassBEpilogue<T, FWD> epi(P, c0 + threadIdx.x % W);
         auto dst = [&](int n, int w, V v) {
             if (w < wv) {
                 if constexpr (EPI)
